@@ -145,9 +145,12 @@ static void launch_cz(const Buffers& in, Buffers& out, uint64_t n, double eps, L
 void check_device_error() {
     if (capturing()) return;
     unsigned v = 0;
-    SQ_CUDA(cudaMemcpyAsync(&v, device_error_word(), 4, cudaMemcpyDeviceToHost, stream()));
-    SQ_CUDA(cudaStreamSynchronize(stream()));
+    if (!mailed_error(&v)) {  // else the last read-back brought it along
+        SQ_CUDA(cudaMemcpyAsync(&v, device_error_word(), 4, cudaMemcpyDeviceToHost, stream()));
+        SQ_CUDA(cudaStreamSynchronize(stream()));
+    }
     if (v) {
+        count_launch(0);  // a mailed error word is stale from here on
         SQ_CUDA(cudaMemsetAsync(device_error_word(), 0, 4, stream()));
         if (v & 32u) fail(SQ_ERR_INVALID, "a replayed graph saw other sizes than were recorded; the state is not valid");
         if (v & 64u) fail(SQ_ERR_INVALID, "angle: a register pair has no entry in the angle table");

@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdlib>
+#include <cstddef>
 #include <cstring>
 #include <stdexcept>
 
@@ -139,6 +140,7 @@ static cudaStream_t g_stream = nullptr;
 static int g_sms = 0;
 static int g_device = -1;
 static std::atomic<uint64_t> g_launches{0};
+static bool g_mail_err_fresh = false;  // nothing was launched since a read-back brought the error word (mail_wait)
 
 cudaStream_t stream() {
     if (!g_stream) {
@@ -188,7 +190,10 @@ unsigned int* device_error_word() {
     return g_err_word;
 }
 
-void count_launch(int n) { g_launches += (uint64_t)n; }
+void count_launch(int n) {
+    g_launches += (uint64_t)n;
+    g_mail_err_fresh = false;
+}
 uint64_t launches() { return g_launches.load(); }
 
 // ------------------------------------------------------------------ per-kernel timing
@@ -245,6 +250,92 @@ __global__ void replay_check_kernel(const unsigned char* __restrict__ src, const
         if (src[i] != want.b[i]) atomicOr(err, 32u);
 }
 
+// Read-backs. A split reads one to three small results (counts, flags) before
+// the next launch can be sized, and that round trip is most of a small split's
+// time. They come back through mapped pinned memory: one block (or the last
+// kernel of the operator itself, MailSlot) stores the bytes and the device
+// error word and then a sequence number that the host spins on. Measured per
+// kernel + read-back: 6.8 us, or 8.8 us with the extra block, against 14.2 us
+// for cudaMemcpyAsync into pageable memory and a stream synchronise (and such
+// a copy also queues behind a bulk download on the copy engine).
+struct Mail {
+    unsigned long long seq;
+    unsigned err;
+    unsigned pad;
+    unsigned char b[kMailBytes];
+};
+static_assert(offsetof(Mail, b) == kMailData && offsetof(Mail, err) == kMailErr, "layout shared with mail_post");
+static unsigned char* g_mail_dev = nullptr;
+static Mail* g_mail_host = nullptr;
+static unsigned long long g_mail_seq = 0;
+static unsigned g_mail_err = 0;
+
+__global__ void mail_kernel(const unsigned char* __restrict__ src, unsigned bytes, const unsigned* err,
+                            unsigned char* mail, unsigned long long seq) {
+    unsigned char* b = mail + kMailData;
+    if (((reinterpret_cast<uintptr_t>(src) | bytes) & 3) == 0) {
+        for (unsigned i = threadIdx.x; i < bytes / 4; i += blockDim.x)
+            reinterpret_cast<volatile unsigned*>(b)[i] = reinterpret_cast<const unsigned*>(src)[i];
+    } else {
+        for (unsigned i = threadIdx.x; i < bytes; i += blockDim.x) reinterpret_cast<volatile unsigned char*>(b)[i] = src[i];
+    }
+    __threadfence_system();
+    __syncthreads();
+    if (threadIdx.x == 0) mail_seal(mail, err, seq);
+}
+
+static unsigned long long mail_next() {
+    if (!g_mail_host) {
+        SQ_CUDA(cudaHostAlloc((void**)&g_mail_host, sizeof(Mail), cudaHostAllocMapped));
+        memset(g_mail_host, 0, sizeof(Mail));
+        SQ_CUDA(cudaHostGetDevicePointer((void**)&g_mail_dev, g_mail_host, 0));
+    }
+    return ++g_mail_seq;
+}
+
+static void log_read(const void* v, size_t bytes) {
+    if (g_replay.mode != RP_RECORD) return;
+    const unsigned char* b = static_cast<const unsigned char*>(v);
+    g_replay.log.insert(g_replay.log.end(), b, b + bytes);
+}
+
+// Waits for letter `seq`. The stream is asked now and then whether it failed,
+// so a fault is reported instead of waited for.
+static void mail_wait(unsigned long long seq, void* dst, size_t bytes) {
+    for (unsigned spins = 1; __atomic_load_n(&g_mail_host->seq, __ATOMIC_ACQUIRE) != seq; ++spins) {
+        if (spins & 0x3fffu) continue;
+        const cudaError_t q = cudaStreamQuery(stream());
+        if (q == cudaErrorNotReady) continue;
+        SQ_CUDA(q);
+        if (__atomic_load_n(&g_mail_host->seq, __ATOMIC_ACQUIRE) != seq) fail(SQ_ERR_CUDA, "read-back: no letter");
+        break;
+    }
+    memcpy(dst, g_mail_host->b, bytes);
+    g_mail_err = g_mail_host->err;
+    g_mail_err_fresh = true;
+    log_read(dst, bytes);
+}
+
+MailSlot mail_slot() {
+    MailSlot m;
+    if (capturing()) return m;  // a replayed kernel must not write to the host: host_read's check instead
+    m.seq = mail_next();
+    m.mail = g_mail_dev;
+    m.err = device_error_word();
+    return m;
+}
+
+void mail_read(const MailSlot& m, void* dst, const void* dev, size_t bytes) {
+    if (m.mail) mail_wait(m.seq, dst, bytes);
+    else host_read(dst, dev, bytes);
+}
+
+bool mailed_error(unsigned* err) {
+    if (!g_mail_err_fresh) return false;
+    *err = g_mail_err;
+    return true;
+}
+
 void host_read(void* dst, const void* src, size_t bytes) {
     ReplayState& r = g_replay;
     if (r.mode == RP_CAPTURE) {
@@ -260,12 +351,18 @@ void host_read(void* dst, const void* src, size_t bytes) {
         count_launch();
         return;
     }
+    if (bytes <= kMailBytes) {
+        const unsigned long long seq = mail_next();
+        mail_kernel<<<1, 128, 0, stream()>>>(static_cast<const unsigned char*>(src), (unsigned)bytes,
+                                             device_error_word(), g_mail_dev, seq);
+        SQ_CUDA(cudaGetLastError());
+        count_launch();
+        mail_wait(seq, dst, bytes);
+        return;
+    }
     SQ_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream()));
     SQ_CUDA(cudaStreamSynchronize(stream()));
-    if (r.mode == RP_RECORD) {
-        const unsigned char* b = static_cast<const unsigned char*>(dst);
-        r.log.insert(r.log.end(), b, b + bytes);
-    }
+    log_read(dst, bytes);
 }
 
 void host_decision(void* v, size_t bytes) {

@@ -283,6 +283,36 @@ bool capturing();
 // a read-back (logged when recording); under capture the logged bytes, with a
 // device-side check that the replay produces the same.
 void host_read(void* dst, const void* src, size_t bytes);
+// Read-backs through mapped pinned memory: `bytes` of payload at kMailData,
+// the device error word at kMailErr, and a sequence number at 0 written last.
+constexpr size_t kMailBytes = 8192;
+constexpr unsigned kMailErr = 8, kMailData = 16;
+struct MailSlot {
+    unsigned char* mail = nullptr;  // null under capture: nothing is posted
+    const unsigned* err = nullptr;
+    unsigned long long seq = 0;
+};
+// A slot for the next kernel, which posts its 8-byte result with mail_post;
+// mail_read waits for it (under capture: host_read of `dev`, where the kernel
+// leaves the result as well). One slot is open at a time.
+MailSlot mail_slot();
+void mail_read(const MailSlot& m, void* dst, const void* dev, size_t bytes);
+// The device error word as the last read-back saw it, when nothing has been
+// launched since.
+bool mailed_error(unsigned* err);
+#ifdef __CUDACC__
+__device__ __forceinline__ void mail_seal(unsigned char* mail, const unsigned* err, unsigned long long seq) {
+    *reinterpret_cast<volatile unsigned*>(mail + kMailErr) = *reinterpret_cast<const volatile unsigned*>(err);
+    __threadfence_system();
+    *reinterpret_cast<volatile unsigned long long*>(mail) = seq;
+}
+// One thread, after every store and error flag of the operator is visible to it.
+__device__ __forceinline__ void mail_post(const MailSlot& m, unsigned long long v) {
+    if (!m.mail) return;
+    *reinterpret_cast<volatile unsigned long long*>(m.mail + kMailData) = v;
+    mail_seal(m.mail, m.err, m.seq);
+}
+#endif
 // A host-side choice (autotuning, timing-dependent paths): logged when
 // recording, taken from the log under capture.
 void host_decision(void* v, size_t bytes);
