@@ -61,6 +61,10 @@ __device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_doub
 __device__ __forceinline__ double2 cmul2(double2 a, double2 b) {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
+__device__ __forceinline__ bool finite2(double2 a) {
+    const unsigned hx = (unsigned)__double2hiint(a.x), hy = (unsigned)__double2hiint(a.y);
+    return (hx & 0x7ff00000u) != 0x7ff00000u && (hy & 0x7ff00000u) != 0x7ff00000u;
+}
 __device__ __forceinline__ bool keep_amp(double2 a, double eps) { return sq_keep_amp(a.x, a.y, eps); }
 // Store of a or -a (the bits of a * -1.0 for every non-NaN a) as integer
 // bits: a negation kept in double registers would be issued as an FP64 add.
@@ -425,6 +429,7 @@ struct EmitArgs {
     double eps;
     double sign2pi;            // CondRot: +-2*pi
     double2 m[4];
+    int real;                  // m (no mtable) has no imaginary parts
     const double2* mtable;     // CondRot_General_Bool: 4 matrix elements per input value
     const double2* umat;       // Rot_GeneralUnitary: S x S row-major
     int udag;                  // Rot_GeneralUnitary: apply the conjugate transpose
@@ -503,8 +508,8 @@ __device__ __forceinline__ void store_out_sign(const EmitArgs& a, unsigned long 
 }
 
 __device__ __forceinline__ double as_rational(uint64_t v, unsigned w) {
-    if (w >= 64) return v * 1.0 / 2 / 9223372036854775808.0;
-    return 1.0 * v / (double)(1ull << w);
+    // v / 2^w: a product with the power of two rounds as the division does
+    return (double)v * __longlong_as_double((long long)(1023 - (int)w) << 52);
 }
 
 // Member `pos` of the grouped order: its target value and amplitude. The
@@ -546,7 +551,6 @@ template <int K>
 __device__ __forceinline__ void pair_math(const EmitArgs& a, const uint64_t (&k0)[K], double2 az, double2 ao,
                                           bool has_z, bool has_o, double2& rz, double2& ro, bool& kz, bool& ko) {
     {
-        const double2 zero = make_double2(0.0, 0.0);
         if (a.mode == GM_HADAMARD_BOOL) {
             const double s = a.sqrt2inv;
             if (has_z && has_o) {
@@ -568,7 +572,19 @@ __device__ __forceinline__ void pair_math(const EmitArgs& a, const uint64_t (&k0
                 m2 = mt[2];
                 m3 = mt[3];
             }
-            if (has_z && has_o) {
+            if (a.real && finite2(az) && finite2(ao)) {
+                // a real matrix (RY, the QDA rotation): the products with its
+                // zero imaginary parts leave finite values as they are (only
+                // the sign of a zero may differ); 4 or 12 FP64 operations
+                // instead of 12 or 28
+                if (has_z && has_o) {
+                    rz = cadd(cscale(az, m0.x), cscale(ao, m1.x));
+                    ro = cadd(cscale(az, m2.x), cscale(ao, m3.x));
+                } else {
+                    rz = cscale(has_z ? az : ao, has_z ? m0.x : m1.x);
+                    ro = cscale(has_z ? az : ao, has_z ? m2.x : m3.x);
+                }
+            } else if (has_z && has_o) {
                 rz = cadd(cmul2(az, m0), cmul2(ao, m1));
                 ro = cadd(cmul2(az, m2), cmul2(ao, m3));
             } else if (has_z) {
@@ -582,10 +598,16 @@ __device__ __forceinline__ void pair_math(const EmitArgs& a, const uint64_t (&k0
             const double rot = as_rational(fget<K>(k0, a.aux), a.aux.width) * a.sign2pi;
             double sn, cs;
             sincos(rot, &sn, &cs);
-            if (!has_z) az = zero;
-            if (!has_o) ao = zero;
-            rz = csub(cscale(az, cs), cscale(ao, sn));
-            ro = cadd(cscale(az, sn), cscale(ao, cs));
+            if (has_z && has_o) {
+                rz = csub(cscale(az, cs), cscale(ao, sn));
+                ro = cadd(cscale(az, sn), cscale(ao, cs));
+            } else if (has_z) {  // the reference's zero partner adds nothing
+                rz = cscale(az, cs);
+                ro = cscale(az, sn);
+            } else {
+                rz = cscale(ao, -sn);
+                ro = cscale(ao, cs);
+            }
         }
         kz = keep_amp(rz, a.eps);
         ko = keep_amp(ro, a.eps);
@@ -2766,18 +2788,27 @@ static Grouping group_by_hash(State& s, const GroupSpec& gs, uint64_t* dg, uint6
 
 // ------------------------------------------------------------------ pair splits by partner lookup
 // A 1-bit split pairs each entry with the entry whose key differs in the
-// target bit alone. Instead of grouping (hash buckets or a sort of the keys
-// without the bit), the entries that pass the conditions go into an
-// open-addressing table by their whole key (keys are unique), and every
-// entry looks its partner up: the member with bit 0 of a pair, or a member
-// without a partner, writes the pair's outputs (pair_math, the arithmetic of
-// the grouped path); the member with bit 1 of a pair writes nothing; entries
-// that fail the conditions are copied. A slot is (fingerprint 24 | index + 1),
-// zero empty; the table holds at least twice the entries, so every probe
-// sequence ends at an empty slot.
+// target bit alone (keys are unique). No grouping: members of a pair meet in
+// an open-addressing table on the key without the target bit. The first to
+// arrive leaves its index in the slot; the second finds it there, knows both
+// members and writes the pair's outputs at once (pair_math, the arithmetic of
+// the grouped path). Entries that met nobody are written by a last pass, and
+// so are the entries that fail the conditions (copied). A slot is
+// (fingerprint 24 | index + 1), zero empty; the table holds at least twice the
+// entries, so every probe sequence ends at an empty slot.
+//
+// What bounds it: the random table accesses (2^21 random 64-bit
+// compare-and-swaps take 40 us, as many random loads 15 us; at 2^24, where the
+// table no longer fits L2, 555 and 231 us) and the output reservations (0.7 ns
+// per atomic on one address). A build pass followed by a lookup pass costs two
+// random accesses and one key comparison per entry more: 179 us of kernels per
+// split of a dense 2^21-entry state against 125 us (flags 6, clear 6, claim 95,
+// lone 4, event overheads included) in this form.
 struct PairTable {
     unsigned long long* slots;
     unsigned long long mask;  // capacity - 1
+    unsigned* flags;          // bit 0: a passing entry has target bit 0, bit 1: one has 1
+    unsigned char* met;       // 1: the entry found its partner
 };
 template <int K>
 __device__ __forceinline__ unsigned long long full_key_hash(const uint64_t (&k)[K]) {
@@ -2786,133 +2817,353 @@ __device__ __forceinline__ unsigned long long full_key_hash(const uint64_t (&k)[
     for (int w = 0; w < K; ++w) hv = mix64(hv ^ k[w] ^ (0x632be59bd9b4e019ull * (w + 1)));
     return hv;
 }
-
+// The hash of a key without its target bit.
 template <int K>
-__global__ void __launch_bounds__(256) pair_table_build_kernel(ConstKeyPtrs keys, uint64_t n, DCondSet cond,
-                                                               PairTable t) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        uint64_t k[K];
-        load_key<K>(keys, i, k);
-        if (!cond_ok<K>(k, cond)) continue;
-        const unsigned long long hv = full_key_hash<K>(k);
-        const unsigned long long tag = ((hv >> 40) << 32) | (unsigned long long)(i + 1);
-        unsigned long long slot = hv & t.mask;
-        // at most capacity probes; a lost race re-reads the slot it lost
-        // (filled now), so the loop moves on after at most one retry per slot
-        for (unsigned long long probes = 0; probes <= t.mask;) {
-            const unsigned long long v = t.slots[slot];
-            if (v == 0ull) {
-                if (atomicCAS(&t.slots[slot], 0ull, tag) == 0ull) break;
-                continue;
-            }
-            slot = (slot + 1) & t.mask;
-            ++probes;
-        }
-    }
-}
-
-// The entry index holding key pk, or -1.
-template <int K>
-__device__ __forceinline__ long long pair_find(const PairTable& t, const ConstKeyPtrs& keys, const uint64_t (&pk)[K]) {
-    const unsigned long long hv = full_key_hash<K>(pk);
-    const unsigned long long fp = hv >> 40;
-    unsigned long long slot = hv & t.mask;
-    for (unsigned long long probes = 0; probes <= t.mask; ++probes) {
-        const unsigned long long v = __ldg(t.slots + slot);
-        if (v == 0ull) return -1;
-        if ((v >> 32) == fp) {
-            const unsigned long long j = (v & 0xffffffffull) - 1ull;
-            bool eq = true;
+__device__ __forceinline__ unsigned long long pair_hash(const uint64_t (&k)[K], unsigned tw, uint64_t bit) {
+    uint64_t g[K];
 #pragma unroll
-            for (int w = 0; w < K; ++w) eq = eq && (__ldg(keys.w[w] + j) == pk[w]);
-            if (eq) return (long long)j;
-        }
-        slot = (slot + 1) & t.mask;
-    }
-    return -1;
+    for (int w = 0; w < K; ++w) g[w] = (unsigned)w == tw ? k[w] & ~bit : k[w];
+    return full_key_hash<K>(g);
+}
+template <int K>
+__device__ __forceinline__ bool is_partner(const ConstKeyPtrs& keys, unsigned long long j, const uint64_t (&k)[K],
+                                           unsigned tw, uint64_t bit) {
+    bool eq = true;
+#pragma unroll
+    for (int w = 0; w < K; ++w) eq = eq && __ldg(keys.w[w] + j) == ((unsigned)w == tw ? k[w] ^ bit : k[w]);
+    return eq;
 }
 
-// One thread per entry; the lanes of a warp reserve their outputs with one
-// atomic, in lane order. Writes nothing past a.capacity (the bound 2n is
-// exact, so that only matters to a graph replayed on other data).
+// Exclusive scan of a count over a CTA in thread order; `total` over the CTA.
+// s: one word per warp. Two barriers, so that s may be reused right away.
+template <int BLOCK>
+__device__ __forceinline__ unsigned block_rank(unsigned c, unsigned* s, unsigned& total) {
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    unsigned inc = c;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const unsigned v = __shfl_up_sync(0xffffffffu, inc, d);
+        if (lane >= (unsigned)d) inc += v;
+    }
+    if (lane == 31u) s[warp] = inc;
+    __syncthreads();
+    unsigned pre = 0, tot = 0;
+#pragma unroll
+    for (int w = 0; w < BLOCK / 32; ++w) {
+        const unsigned v = s[w];
+        if ((unsigned)w < warp) pre += v;
+        tot += v;
+    }
+    __syncthreads();
+    total = tot;
+    return pre + inc - c;
+}
+
+// One reservation on the output cursor per CTA (a reservation per warp put
+// 65,536 same-address atomics, 46 us, into a 2^21-entry split). Returns the
+// calling thread's first output; `fits` is uniform over the CTA.
+template <int BLOCK>
+__device__ __forceinline__ unsigned long long block_reserve(const EmitArgs& a, unsigned c, unsigned* s,
+                                                            unsigned long long* s_base, bool& fits) {
+    unsigned total;
+    const unsigned rank = block_rank<BLOCK>(c, s, total);
+    if (threadIdx.x == 0) *s_base = total ? atomicAdd(a.cursor, (unsigned long long)total) : 0ull;
+    __syncthreads();
+    const unsigned long long base = *s_base;
+    fits = base + total <= a.capacity;
+    __syncthreads();
+    return base + rank;
+}
+
 template <int K>
-__global__ void __launch_bounds__(256) pair_partner_emit_kernel(const __grid_constant__ EmitArgs a, uint64_t n,
-                                                                DCondSet cond, PairTable t) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    const unsigned lane = threadIdx.x & 31u;
+__device__ __forceinline__ void store_pair(const EmitArgs& a, unsigned long long o, uint64_t (&k)[K], double2 rz,
+                                           double2 ro, bool kz, bool ko) {
+    if (kz) {
+        fset<K>(k, a.target, 0);
+        store_out<K>(a, o++, k, rz);
+    }
+    if (ko) {
+        fset<K>(k, a.target, 1);
+        store_out<K>(a, o, k, ro);
+    }
+}
+
+// Which values the target bit takes among the passing entries: while it is
+// constant (a flag or ancilla still at |0>, as after AddRegister) no entry
+// has a partner, and the table is neither cleared nor filled. CTAs stop
+// reading once both values were seen, which is after their first entries
+// unless the bit is constant. `words`: the key words the conditions and the
+// target use.
+template <int K>
+__global__ void __launch_bounds__(256) pair_flags_kernel(ConstKeyPtrs keys, uint64_t n,
+                                                         const __grid_constant__ DCondSet cond, unsigned words,
+                                                         Field tgt, unsigned* flags) {
+    const uint64_t stride = (uint64_t)gridDim.x * 1024u;
+    for (uint64_t b = (uint64_t)blockIdx.x * 1024u; b < n; b += stride) {
+        const unsigned seen = *reinterpret_cast<volatile unsigned*>(flags);
+        unsigned f = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint64_t i = b + (uint64_t)q * 256u + threadIdx.x;
+            if (i >= n) continue;
+            uint64_t k[K];
+#pragma unroll
+            for (int w = 0; w < K; ++w) k[w] = ((words >> w) & 1u) ? keys.w[w][i] : 0ull;
+            if (cond_ok<K>(k, cond)) f |= fget<K>(k, tgt) ? 2u : 1u;
+        }
+        const unsigned all = (__syncthreads_or(f & 1u) ? 1u : 0u) | (__syncthreads_or(f & 2u) ? 2u : 0u);
+        if (threadIdx.x == 0 && (all & ~seen)) atomicOr(flags, all);
+        if (all == 3u || __syncthreads_or(seen == 3u)) break;
+    }
+}
+
+// Clears the table and the met marks when there can be partners.
+static __global__ void __launch_bounds__(256) pair_clear_kernel(PairTable t, uint64_t met16) {
+    if (*t.flags != 3u) return;
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, n16 = (t.mask + 1) / 2;
+    const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n16 + met16; i += stride) {
+        if (i < n16) reinterpret_cast<uint4*>(t.slots)[i] = z;
+        else reinterpret_cast<uint4*>(t.met)[i - n16] = z;
+    }
+}
+
+// Every passing entry goes into the table or finds its partner there; a pair
+// is written by the CTA of its second member. The pairs a CTA finds are
+// listed in shared memory and then computed by consecutive threads: the FP64
+// pipe (2 lanes per SM and clock) takes as long for a warp with every second
+// lane active as for a full one. Failing entries are copied. ITEMS entries
+// per thread keep their table accesses in flight together and share one
+// output reservation.
+template <int K, int ITEMS>
+__global__ void __launch_bounds__(256) pair_claim_kernel(const __grid_constant__ EmitArgs a, uint64_t n,
+                                                         const __grid_constant__ DCondSet cond, PairTable t) {
+    __shared__ unsigned s_w[8];
+    __shared__ unsigned long long s_base;
+    __shared__ unsigned s_z[256 * ITEMS], s_o[256 * ITEMS];  // the pairs: entry with target bit 0, with 1
+    if (*t.flags != 3u) return;
+    const unsigned tw = a.target.word;
     const uint64_t bit = 1ull << a.target.shift;
-    for (uint64_t gb = (uint64_t)blockIdx.x * blockDim.x; gb < n; gb += stride) {  // warp-uniform trips
-        const uint64_t i = gb + threadIdx.x;
-        const bool valid = i < n;
-        uint64_t k[K];
-        double2 rz = make_double2(0.0, 0.0), ro = make_double2(0.0, 0.0);
-        bool kz = false, ko = false, copy = false;
-        if (valid) {
-            load_key<K>(a.in_keys, i, k);
-            const double2 ai = a.in_amp[i];
-            if (!cond_ok<K>(k, cond)) {
-                copy = true;
-                rz = ai;
-            } else {
-                const bool one = (k[a.target.word] & bit) != 0ull;
-                uint64_t pk[K];
+    const uint64_t stride = (uint64_t)gridDim.x * (256u * ITEMS);
+    for (uint64_t b = (uint64_t)blockIdx.x * (256u * ITEMS); b < n; b += stride) {
+        unsigned copy = 0, found = 0;  // bit q: item q fails the conditions / met its partner
+        unsigned partner[ITEMS], one = 0;
+        {
+            uint64_t k[ITEMS][K];
+            unsigned long long slot[ITEMS], tag[ITEMS], v[ITEMS];
+            unsigned pass = 0;
 #pragma unroll
-                for (int w = 0; w < K; ++w) pk[w] = k[w];
-                pk[a.target.word] ^= bit;
-                const long long j = pair_find<K>(t, a.in_keys, pk);
-                if (!(one && j >= 0)) {  // the bit-0 member of a pair, or a lone member
-                    const double2 aj = j >= 0 ? a.in_amp[j] : make_double2(0.0, 0.0);
-                    const double2 az = one ? aj : ai, ao = one ? ai : aj;
-                    pair_math<K>(a, k, az, ao, !one || j >= 0, one || j >= 0, rz, ro, kz, ko);
+            for (int q = 0; q < ITEMS; ++q) {
+                const uint64_t i = b + (uint64_t)q * 256u + threadIdx.x;
+                if (i < n) load_key<K>(a.in_keys, (unsigned)i, k[q]);
+            }
+#pragma unroll
+            for (int q = 0; q < ITEMS; ++q) {
+                const uint64_t i = b + (uint64_t)q * 256u + threadIdx.x;
+                if (i >= n) continue;
+                if (!cond_ok<K>(k[q], cond)) {
+                    copy |= 1u << q;
+                    t.met[i] = 1;
+                    continue;
+                }
+                pass |= 1u << q;
+                const unsigned long long hv = pair_hash<K>(k[q], tw, bit);
+                tag[q] = ((hv >> 40) << 32) | (unsigned long long)(i + 1);
+                slot[q] = hv & t.mask;
+                v[q] = atomicCAS(&t.slots[slot[q]], 0ull, tag[q]);
+            }
+#pragma unroll
+            for (int q = 0; q < ITEMS; ++q) {
+                if (!((pass >> q) & 1u)) continue;
+                // at most capacity probes; the table is at most half full
+                for (unsigned long long probes = 0; v[q] != 0ull && probes <= t.mask; ++probes) {
+                    if ((v[q] >> 32) == (tag[q] >> 32) &&
+                        is_partner<K>(a.in_keys, (v[q] & 0xffffffffull) - 1ull, k[q], tw, bit)) {
+                        partner[q] = (unsigned)(v[q] & 0xffffffffull) - 1u;
+                        found |= 1u << q;
+                        if (kword<K>(k[q], tw) & bit) one |= 1u << q;
+                        t.met[b + (uint64_t)q * 256u + threadIdx.x] = 1;
+                        t.met[partner[q]] = 1;
+                        break;
+                    }
+                    slot[q] = (slot[q] + 1) & t.mask;
+                    v[q] = atomicCAS(&t.slots[slot[q]], 0ull, tag[q]);
                 }
             }
         }
-        const unsigned c = copy ? 1u : (unsigned)kz + (unsigned)ko;
-        unsigned inc = c;
+        unsigned pairs;
+        unsigned at = block_rank<256>(__popc(found), s_w, pairs);
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const unsigned v = __shfl_up_sync(0xffffffffu, inc, d);
-            if (lane >= (unsigned)d) inc += v;
+        for (int q = 0; q < ITEMS; ++q) {
+            if (!((found >> q) & 1u)) continue;
+            const unsigned i = (unsigned)(b + (uint64_t)q * 256u + threadIdx.x);
+            const bool o = (one >> q) & 1u;
+            s_z[at] = o ? partner[q] : i;
+            s_o[at++] = o ? i : partner[q];
         }
-        const unsigned total = __shfl_sync(0xffffffffu, inc, 31);
-        unsigned long long base = 0;
-        if (lane == 31 && total) base = atomicAdd(a.cursor, (unsigned long long)total);
-        base = __shfl_sync(0xffffffffu, base, 31);
-        if (!valid || c == 0 || base + total > a.capacity) continue;
-        unsigned long long o = base + (inc - c);
-        if (copy) {
-            store_out<K>(a, o, k, rz);
-            continue;
+        __syncthreads();
+        if (__syncthreads_or(copy)) {
+            bool fits;
+            unsigned long long o = block_reserve<256>(a, __popc(copy), s_w, &s_base, fits);
+#pragma unroll
+            for (int q = 0; q < ITEMS; ++q) {
+                if (!fits || !((copy >> q) & 1u)) continue;
+                const uint64_t i = b + (uint64_t)q * 256u + threadIdx.x;
+                uint64_t k[K];
+                load_key<K>(a.in_keys, (unsigned)i, k);
+                store_out<K>(a, o++, k, a.in_amp[i]);
+            }
         }
-        if (kz) {
-            fset<K>(k, a.target, 0);
-            store_out<K>(a, o++, k, rz);
+        for (unsigned p0 = 0; p0 < pairs; p0 += 256u) {
+            const unsigned p = p0 + threadIdx.x;
+            uint64_t k[K];
+            double2 rz, ro;
+            bool kz = false, ko = false;
+            if (p < pairs) {
+                const unsigned z = s_z[p];
+                load_key<K>(a.in_keys, z, k);
+                pair_math<K>(a, k, a.in_amp[z], a.in_amp[s_o[p]], true, true, rz, ro, kz, ko);
+            }
+            bool fits;
+            const unsigned long long o = block_reserve<256>(a, (unsigned)kz + (unsigned)ko, s_w, &s_base, fits);
+            if (fits && (kz || ko)) store_pair<K>(a, o, k, rz, ro, kz, ko);
         }
-        if (ko) {
-            fset<K>(k, a.target, 1);
-            store_out<K>(a, o, k, ro);
+        __syncthreads();
+    }
+}
+
+// The entries not written by the claim pass: the passing entries that met no
+// partner or, when the target bit is constant (no claim pass ran), every
+// entry, failing ones copied.
+template <int K>
+__global__ void __launch_bounds__(256) pair_lone_kernel(const __grid_constant__ EmitArgs a, uint64_t n,
+                                                        const __grid_constant__ DCondSet cond, PairTable t) {
+    __shared__ unsigned s_w[8];
+    __shared__ unsigned long long s_base;
+    const bool claimed = *t.flags == 3u;
+    const unsigned tw = a.target.word;
+    const uint64_t bit = 1ull << a.target.shift;
+    const uint64_t stride = (uint64_t)gridDim.x * 1024u;
+    for (uint64_t b0 = (uint64_t)blockIdx.x * 1024u; b0 < n; b0 += stride) {
+        unsigned mine = 0;  // bit q: entry b0 + 256 q + thread is left
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint64_t i = b0 + (uint64_t)q * 256u + threadIdx.x;
+            if (i < n && !(claimed && t.met[i])) mine |= 1u << q;
+        }
+        if (!__syncthreads_or(mine)) continue;
+        for (int q = 0; q < 4; ++q) {
+            const uint64_t i = b0 + (uint64_t)q * 256u + threadIdx.x;
+            uint64_t k[K];
+            double2 rz = make_double2(0.0, 0.0), ro = rz;
+            bool kz = false, ko = false, copy = false;
+            if ((mine >> q) & 1u) {
+                load_key<K>(a.in_keys, (unsigned)i, k);
+                const double2 ai = a.in_amp[i];
+                copy = !cond_ok<K>(k, cond);
+                if (copy) {
+                    rz = ai;
+                } else {
+                    const bool one = (kword<K>(k, tw) & bit) != 0ull;
+                    const double2 zero = make_double2(0.0, 0.0);
+                    pair_math<K>(a, k, one ? zero : ai, one ? ai : zero, !one, one, rz, ro, kz, ko);
+                }
+            }
+            bool fits;
+            const unsigned long long o = block_reserve<256>(a, copy ? 1u : (unsigned)kz + (unsigned)ko, s_w, &s_base, fits);
+            if (!fits) continue;
+            if (copy) store_out<K>(a, o, k, rz);
+            else if (kz || ko) store_pair<K>(a, o, k, rz, ro, kz, ko);
         }
     }
 }
 
-// Pair split by partner lookup: table build, one emit pass with reserved
-// outputs (at most 2N: two per passing entry, one per copied entry).
+// The whole split of a small state in one CTA: the table lives in shared
+// memory, members of a pair learn of each other there, and the outputs are
+// written in entry order with their number posted to the host by the same
+// launch. One launch and its read-back instead of a table clear, a build, a
+// cursor clear, an emit and a copy.
+constexpr unsigned kPairSmallMax = 4096;
+constexpr unsigned kPairFailed = 0xffffffffu;
+template <int K, int BLOCK>
+__global__ void __launch_bounds__(BLOCK) pair_small_kernel(const __grid_constant__ EmitArgs a, unsigned n,
+                                                          const __grid_constant__ DCondSet cond, unsigned cap,
+                                                          const __grid_constant__ MailSlot mail) {
+    extern __shared__ unsigned s_pair[];  // cap slots (entry + 1) | n mates (entry + 1)
+    unsigned* table = s_pair;
+    unsigned* mate = s_pair + cap;
+    __shared__ unsigned s_w[32];
+    const unsigned tid = threadIdx.x;
+    const unsigned tw = a.target.word;
+    const uint64_t bit = 1ull << a.target.shift;
+    for (unsigned i = tid; i < cap + n; i += (unsigned)BLOCK) s_pair[i] = 0u;
+    __syncthreads();
+    for (unsigned e = tid; e < n; e += (unsigned)BLOCK) {
+        uint64_t k[K];
+        load_key<K>(a.in_keys, e, k);
+        if (!cond_ok<K>(k, cond)) {
+            mate[e] = kPairFailed;
+            continue;
+        }
+        unsigned slot = (unsigned)pair_hash<K>(k, tw, bit) & (cap - 1u);
+        for (unsigned probes = 0; probes < cap; ++probes) {  // at most half full: ends at an empty slot
+            const unsigned old = atomicCAS(&table[slot], 0u, e + 1u);
+            if (old == 0u) break;
+            if (is_partner<K>(a.in_keys, old - 1u, k, tw, bit)) {
+                mate[e] = old;
+                mate[old - 1u] = e + 1u;
+                break;
+            }
+            slot = (slot + 1u) & (cap - 1u);
+        }
+    }
+    __syncthreads();
+    unsigned long long base = 0;
+    for (unsigned b = 0; b < n; b += (unsigned)BLOCK) {
+        const unsigned e = b + tid;
+        uint64_t k[K];
+        double2 rz = make_double2(0.0, 0.0), ro = rz;
+        bool kz = false, ko = false, copy = false;
+        if (e < n) {
+            const unsigned m = mate[e];
+            load_key<K>(a.in_keys, e, k);
+            const bool one = (kword<K>(k, tw) & bit) != 0ull;
+            if (m == kPairFailed) {
+                copy = true;
+                rz = a.in_amp[e];
+            } else if (!(one && m)) {  // the bit-0 member of a pair, or a lone member
+                const double2 ai = a.in_amp[e], aj = m ? a.in_amp[m - 1u] : make_double2(0.0, 0.0);
+                pair_math<K>(a, k, one ? aj : ai, one ? ai : aj, !one || m, one || m, rz, ro, kz, ko);
+            }
+        }
+        unsigned total;
+        const unsigned long long o = base + block_rank<BLOCK>(copy ? 1u : (unsigned)kz + (unsigned)ko, s_w, total);
+        base += total;
+        if (copy) store_out<K>(a, o, k, rz);
+        else if (kz || ko) store_pair<K>(a, o, k, rz, ro, kz, ko);
+    }
+    if (tid == 0) {
+        *a.cursor = base;
+        mail_post(mail, base);
+    }
+}
+
+static unsigned cond_words(const DCondSet& c) {
+    unsigned m = 0;
+    for (uint32_t i = 0; i < c.n; ++i) m |= 1u << c.c[i].word;
+    return m;
+}
+
+// Pair split by partner lookup; outputs at most 2N (two per passing entry,
+// one per copied entry). Up to kPairSmallMax entries (48 KB of shared memory
+// for table and mates) one CTA does everything: a split of a 256-entry state
+// takes 20 us from call to call against 36 us for the launches of the table
+// path; above, one SM's share of the work is the longer time.
 template <int K>
 static void run_pair_partner(State& s, const GroupSpec& gs, EmitArgs& ea) {
     const uint64_t N = s.n;
     cudaStream_t st = stream();
-    uint64_t cap = 1024;
-    while (cap < 2 * N) cap <<= 1;
-    PairTable t;
-    t.slots = (unsigned long long*)ws().get(WS_PAIR_TABLE, cap * 8);
-    t.mask = cap - 1;
-    SQ_CUDA(cudaMemsetAsync(t.slots, 0, cap * 8, st));
     const DCondSet dc = gs.cond;
-    prof_begin("pair_table_build");
-    pair_table_build_kernel<K><<<grid_for(N, 256, 8), 256, 0, st>>>(ea.in_keys, N, dc, t);
-    prof_end((double)N * 8.0 * K + (double)cap * 8);
-    SQ_CUDA(cudaGetLastError());
     const uint64_t capT = 2 * N;
     ensure_buffers(s.spare, capT, regtable().k, 0);
     for (int w = 0; w < SQ_KMAX; ++w) ea.out_keys.w[w] = s.spare.keys[w];
@@ -2920,13 +3171,49 @@ static void run_pair_partner(State& s, const GroupSpec& gs, EmitArgs& ea) {
     unsigned long long* cur = (unsigned long long*)ws().get(WS_CURSOR, 64);
     ea.cursor = cur;
     ea.capacity = capT;
-    SQ_CUDA(cudaMemsetAsync(cur, 0, 8, st));
-    prof_begin("emit_pair_partner");
-    pair_partner_emit_kernel<K><<<grid_for(N, 256, 8), 256, 0, st>>>(ea, N, dc, t);
-    prof_end((double)N * (8.0 * K + 16));
-    SQ_CUDA(cudaGetLastError());
+    uint64_t cap = N <= kPairSmallMax ? 32 : 1024;
+    while (cap < 2 * N) cap <<= 1;
     unsigned long long T = 0;
-    host_read(&T, cur, 8);
+    if (N <= kPairSmallMax) {
+        const MailSlot mail = mail_slot();
+        prof_begin("pair_small");
+        static bool smem_set = false;
+        if (!smem_set) {
+            SQ_CUDA(cudaFuncSetAttribute(pair_small_kernel<K, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(3 * kPairSmallMax * 4)));
+            smem_set = true;
+        }
+        // up to 256 entries a smaller CTA starts and synchronises faster
+        if (N <= 256) pair_small_kernel<K, 256><<<1, 256, (cap + N) * 4, st>>>(ea, (unsigned)N, dc, (unsigned)cap, mail);
+        else pair_small_kernel<K, 1024><<<1, 1024, (cap + N) * 4, st>>>(ea, (unsigned)N, dc, (unsigned)cap, mail);
+        prof_end((double)N * (8.0 * K + 16));
+        SQ_CUDA(cudaGetLastError());
+        mail_read(mail, &T, cur, 8);
+    } else {
+        PairTable t;
+        const uint64_t met16 = (N + 15) / 16;
+        t.slots = (unsigned long long*)ws().get(WS_PAIR_TABLE, cap * 8 + met16 * 16);
+        t.mask = cap - 1;
+        t.met = (unsigned char*)(t.slots + cap);
+        t.flags = (unsigned*)(cur + 1);
+        SQ_CUDA(cudaMemsetAsync(cur, 0, 16, st));
+        prof_begin("pair_flags");
+        pair_flags_kernel<K><<<grid_for(N, 1024, 4), 256, 0, st>>>(ea.in_keys, N, dc, cond_words(dc) | (1u << gs.target.word),
+                                                                  gs.target, t.flags);
+        prof_end();
+        prof_begin("pair_clear");
+        pair_clear_kernel<<<grid_for(cap / 2, 256, 8), 256, 0, st>>>(t, met16);
+        prof_end();
+        prof_begin("pair_claim");
+        constexpr int ITEMS = K <= 2 ? 4 : K <= 4 ? 2 : 1;
+        pair_claim_kernel<K, ITEMS><<<grid_for((N + ITEMS - 1) / ITEMS, 256, 8), 256, 0, st>>>(ea, N, dc, t);
+        prof_end((double)N * (8.0 * K + 16));
+        prof_begin("pair_lone");
+        pair_lone_kernel<K><<<grid_for(N, 1024, 8), 256, 0, st>>>(ea, N, dc, t);
+        prof_end();
+        SQ_CUDA(cudaGetLastError());
+        host_read(&T, cur, 8);
+    }
     if (T > capT) fail(SQ_ERR_CAPACITY, "pair split wrote past its bound");
     prof_add_bytes_last((double)T * (8 * K + 16));
     swap_live_spare(s);
@@ -3040,6 +3327,9 @@ static void set_emit_smem_limits() {
 #undef SQ_SMEM
 }
 
+static int real_matrix(const GroupSpec& g) {
+    return g.mode == GM_ROT && !g.mtable && g.m[0].y == 0.0 && g.m[1].y == 0.0 && g.m[2].y == 0.0 && g.m[3].y == 0.0;
+}
 static bool same_field(const Field& a, const Field& b) {
     return a.word == b.word && a.shift == b.shift && a.width == b.width;
 }
@@ -3086,6 +3376,7 @@ static void run_group(State& s, const GroupSpec& gs) {
             ea.sign2pi = gs.sign * 2 * 3.14159265358979323846;
             for (int i = 0; i < 4; ++i) ea.m[i] = gs.m[i];
             ea.mtable = gs.mtable;
+            ea.real = real_matrix(gs);
             ea.err = device_error_word();
             run_pair_partner<K>(s, gs, ea);
             return;
@@ -3183,6 +3474,7 @@ static void run_group(State& s, const GroupSpec& gs) {
     ea.sign2pi = gs.sign * 2 * 3.14159265358979323846;
     for (int i = 0; i < 4; ++i) ea.m[i] = gs.m[i];
     ea.mtable = gs.mtable;
+    ea.real = real_matrix(gs);
     ea.umat = gs.umat;
     ea.udag = gs.udag;
     ea.varw = gs.varw;
