@@ -427,7 +427,7 @@ struct EmitArgs {
     double extra;              // 1/sqrt(2^n)
     double sqrt2inv;
     double eps;
-    double sign2pi;            // CondRot: +-2*pi
+    int turn_neg;              // CondRot: rotate by minus the angle
     double2 m[4];
     int real;                  // m (no mtable) has no imaginary parts
     const double2* mtable;     // CondRot_General_Bool: 4 matrix elements per input value
@@ -507,9 +507,52 @@ __device__ __forceinline__ void store_out_sign(const EmitArgs& a, unsigned long 
     if (o < a.capacity) store_entry_sign<K>(a.out_keys, a.out_amp, o, k, v, negate);
 }
 
-__device__ __forceinline__ double as_rational(uint64_t v, unsigned w) {
-    // v / 2^w: a product with the power of two rounds as the division does
-    return (double)v * __longlong_as_double((long long)(1023 - (int)w) << 52);
+// cos and sin (x, y) of 2 pi theta / 2^64, in integer arithmetic: an FP64
+// instruction occupies the 2-lane FP64 pipe of an SM for 16 clocks per warp,
+// in which the SM issues 64 integer ones, and the library's double sincos
+// behind a rounded 2 pi v / 2^w made a conditioned rotation FP64-bound (a
+// fan-out of 2^20 entries: 80 us). The angle is an exact
+// fraction of a turn: theta is reduced to the nearest quarter turn plus
+// f = +-u / 8 turn, 0 <= u <= 1, exactly, and the Taylor series of
+// sin(pi/4 u) / u and cos(pi/4 u) in u^2 are summed in 64-bit fixed point
+// (their last four terms in 32-bit), coefficients (pi/4)^k / k! at the scale
+// that the name gives. Relative error below 5 * 2^-64 before the one rounding
+// to double, also near the zeros of sin and cos; sin(fl(2 pi v / 2^w)) is up
+// to 4.4e-16 off.
+__device__ __forceinline__ double2 turn_cos_sin(uint64_t theta) {
+    const unsigned q = (unsigned)((theta + (1ull << 61)) >> 62) & 3u;
+    const long long f = (long long)(theta - ((uint64_t)q << 62));
+    const uint64_t u = f < 0 ? (uint64_t)(-f) : (uint64_t)f;  // u / 2^61, at most 2^61
+    uint64_t t = __umul64hi(u << 2, u << 2);                  // u^2 at 2^62
+    if (t > (1ull << 62) - 1) t = (1ull << 62) - 1;
+    const uint64_t T = t << 2;
+    const unsigned T32 = (unsigned)(T >> 32);
+    constexpr uint64_t kSin64[6] = {0xc90fdaa22168c235ull, 0x14abbce625be52bfull, 0x00a335e33bad570full,
+                                    0x000265a599cc57b1ull, 0x00000541e0d21fbaull, 0x000000078c1d3f7aull};
+    constexpr unsigned kSin68[4] = {0x7a3d0d34u, 0x005beb6eu, 0x0000355eu, 0x00000019u};
+    constexpr uint64_t kCos63[6] = {0x8000000000000000ull, 0x277a79937c8bbcb5ull, 0x020783e1036b5876ull,
+                                    0x000aae9e3f1e5ffdull, 0x00001e1f506891bbull, 0x00000034da3e5441ull};
+    constexpr unsigned kCos64[4] = {0x7e74e28eu, 0x006db894u, 0x00004832u, 0x00000025u};
+    unsigned s32 = kSin68[3], c32 = kCos64[3];
+#pragma unroll
+    for (int k = 2; k >= 0; --k) {
+        s32 = kSin68[k] - __umulhi(s32, T32);
+        c32 = kCos64[k] - __umulhi(c32, T32);
+    }
+    uint64_t s = s32 >> 4, c = c32 >> 1;
+#pragma unroll
+    for (int k = 5; k >= 0; --k) {
+        s = kSin64[k] - __umul64hi(s, T);
+        c = kCos63[k] - __umul64hi(c, T);
+    }
+    // sin = u s: the product of u's leading 64 bits and s keeps its relative accuracy
+    const int lz = u ? __clzll((long long)u) : 0;
+    const long long ym = (long long)(__umul64hi(u << lz, s) >> 1);
+    const double sn = fixed_to_double(f < 0 ? -ym : ym, -60 - lz), cs = fixed_to_double((long long)(c >> 1), -62);
+    const double a = (q & 1u) ? sn : cs, b = (q & 1u) ? cs : sn;  // quarter turns: (c, s), (-s, c), (-c, -s), (s, -c)
+    const unsigned long long na = (q == 1u || q == 2u) ? 0x8000000000000000ull : 0ull, nb = (q & 2u) ? 0x8000000000000000ull : 0ull;
+    return make_double2(__longlong_as_double(__double_as_longlong(a) ^ (long long)na),
+                        __longlong_as_double(__double_as_longlong(b) ^ (long long)nb));
 }
 
 // Member `pos` of the grouped order: its target value and amplitude. The
@@ -595,9 +638,10 @@ __device__ __forceinline__ void pair_math(const EmitArgs& a, const uint64_t (&k0
                 ro = cmul2(ao, m3);
             }
         } else {  // GM_CONDROT: partner amplitude 0 for singletons, as the reference inserts it
-            const double rot = as_rational(fget<K>(k0, a.aux), a.aux.width) * a.sign2pi;
-            double sn, cs;
-            sincos(rot, &sn, &cs);
+            const uint64_t v = fget<K>(k0, a.aux);
+            const uint64_t turn = a.aux.width ? v << (64 - a.aux.width) : 0ull;
+            const double2 r = turn_cos_sin(a.turn_neg ? 0ull - turn : turn);
+            const double cs = r.x, sn = r.y;
             if (has_z && has_o) {
                 rz = csub(cscale(az, cs), cscale(ao, sn));
                 ro = cadd(cscale(az, sn), cscale(ao, cs));
@@ -2919,7 +2963,7 @@ __global__ void __launch_bounds__(256) pair_flags_kernel(ConstKeyPtrs keys, uint
 
 // Clears the table and the met marks when there can be partners.
 static __global__ void __launch_bounds__(256) pair_clear_kernel(PairTable t, uint64_t met16) {
-    if (*t.flags != 3u) return;
+    if ((*t.flags & 3u) != 3u) return;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, n16 = (t.mask + 1) / 2;
     const uint4 z = make_uint4(0u, 0u, 0u, 0u);
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n16 + met16; i += stride) {
@@ -2941,7 +2985,7 @@ __global__ void __launch_bounds__(256) pair_claim_kernel(const __grid_constant__
     __shared__ unsigned s_w[8];
     __shared__ unsigned long long s_base;
     __shared__ unsigned s_z[256 * ITEMS], s_o[256 * ITEMS];  // the pairs: entry with target bit 0, with 1
-    if (*t.flags != 3u) return;
+    if ((*t.flags & 3u) != 3u) return;
     const unsigned tw = a.target.word;
     const uint64_t bit = 1ull << a.target.shift;
     const uint64_t stride = (uint64_t)gridDim.x * (256u * ITEMS);
@@ -3040,7 +3084,7 @@ __global__ void __launch_bounds__(256) pair_lone_kernel(const __grid_constant__ 
                                                         const __grid_constant__ DCondSet cond, PairTable t) {
     __shared__ unsigned s_w[8];
     __shared__ unsigned long long s_base;
-    const bool claimed = *t.flags == 3u;
+    const bool claimed = (*t.flags & 3u) == 3u;
     const unsigned tw = a.target.word;
     const uint64_t bit = 1ull << a.target.shift;
     const uint64_t stride = (uint64_t)gridDim.x * 1024u;
@@ -3083,7 +3127,7 @@ __global__ void __launch_bounds__(256) pair_lone_kernel(const __grid_constant__ 
 // written in entry order with their number posted to the host by the same
 // launch. One launch and its read-back instead of a table clear, a build, a
 // cursor clear, an emit and a copy.
-constexpr unsigned kPairSmallMax = 4096;
+constexpr unsigned kPairSmallMax = 2048;
 constexpr unsigned kPairFailed = 0xffffffffu;
 template <int K, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) pair_small_kernel(const __grid_constant__ EmitArgs a, unsigned n,
@@ -3148,6 +3192,11 @@ __global__ void __launch_bounds__(BLOCK) pair_small_kernel(const __grid_constant
     }
 }
 
+// Above this the target bit is looked at first: two more launches (5 us) for
+// the chance to skip the table (8 to 16 bytes per entry cleared, a random
+// compare-and-swap per entry).
+constexpr uint64_t kPairFlagsMin = 1u << 16;
+
 static unsigned cond_words(const DCondSet& c) {
     unsigned m = 0;
     for (uint32_t i = 0; i < c.n; ++i) m |= 1u << c.c[i].word;
@@ -3155,10 +3204,10 @@ static unsigned cond_words(const DCondSet& c) {
 }
 
 // Pair split by partner lookup; outputs at most 2N (two per passing entry,
-// one per copied entry). Up to kPairSmallMax entries (48 KB of shared memory
-// for table and mates) one CTA does everything: a split of a 256-entry state
-// takes 20 us from call to call against 36 us for the launches of the table
-// path; above, one SM's share of the work is the longer time.
+// one per copied entry). Up to kPairSmallMax entries one CTA does everything:
+// from call to call (RY, one key word) 16 us against 34 through the table at
+// 256 entries, 28 against 45 at 2048; at 4096 one SM's share of the work, 40
+// us, is longer than the table path's 31.
 template <int K>
 static void run_pair_partner(State& s, const GroupSpec& gs, EmitArgs& ea) {
     const uint64_t N = s.n;
@@ -3177,12 +3226,6 @@ static void run_pair_partner(State& s, const GroupSpec& gs, EmitArgs& ea) {
     if (N <= kPairSmallMax) {
         const MailSlot mail = mail_slot();
         prof_begin("pair_small");
-        static bool smem_set = false;
-        if (!smem_set) {
-            SQ_CUDA(cudaFuncSetAttribute(pair_small_kernel<K, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(3 * kPairSmallMax * 4)));
-            smem_set = true;
-        }
         // up to 256 entries a smaller CTA starts and synchronises faster
         if (N <= 256) pair_small_kernel<K, 256><<<1, 256, (cap + N) * 4, st>>>(ea, (unsigned)N, dc, (unsigned)cap, mail);
         else pair_small_kernel<K, 1024><<<1, 1024, (cap + N) * 4, st>>>(ea, (unsigned)N, dc, (unsigned)cap, mail);
@@ -3196,17 +3239,27 @@ static void run_pair_partner(State& s, const GroupSpec& gs, EmitArgs& ea) {
         t.mask = cap - 1;
         t.met = (unsigned char*)(t.slots + cap);
         t.flags = (unsigned*)(cur + 1);
-        SQ_CUDA(cudaMemsetAsync(cur, 0, 16, st));
-        prof_begin("pair_flags");
-        pair_flags_kernel<K><<<grid_for(N, 1024, 4), 256, 0, st>>>(ea.in_keys, N, dc, cond_words(dc) | (1u << gs.target.word),
-                                                                  gs.target, t.flags);
-        prof_end();
-        prof_begin("pair_clear");
-        pair_clear_kernel<<<grid_for(cap / 2, 256, 8), 256, 0, st>>>(t, met16);
-        prof_end();
+        if (N > kPairFlagsMin) {
+            SQ_CUDA(cudaMemsetAsync(cur, 0, 16, st));
+            prof_begin("pair_flags");
+            pair_flags_kernel<K><<<grid_for(N, 1024, 4), 256, 0, st>>>(ea.in_keys, N, dc, cond_words(dc) | (1u << gs.target.word),
+                                                                       gs.target, t.flags);
+            prof_end();
+            prof_begin("pair_clear");
+            pair_clear_kernel<<<grid_for(cap / 2, 256, 8), 256, 0, st>>>(t, met16);
+            prof_end();
+        } else {
+            SQ_CUDA(cudaMemsetAsync(cur, 0, 8, st));
+            SQ_CUDA(cudaMemsetAsync(t.flags, 0xff, 4, st));
+            SQ_CUDA(cudaMemsetAsync(t.slots, 0, cap * 8 + met16 * 16, st));
+        }
         prof_begin("pair_claim");
+        // several entries per thread once that still fills the SMs
         constexpr int ITEMS = K <= 2 ? 4 : K <= 4 ? 2 : 1;
-        pair_claim_kernel<K, ITEMS><<<grid_for((N + ITEMS - 1) / ITEMS, 256, 8), 256, 0, st>>>(ea, N, dc, t);
+        if (N >= (uint64_t)num_sms() * 256 * ITEMS)
+            pair_claim_kernel<K, ITEMS><<<grid_for((N + ITEMS - 1) / ITEMS, 256, 8), 256, 0, st>>>(ea, N, dc, t);
+        else
+            pair_claim_kernel<K, 1><<<grid_for(N, 256, 8), 256, 0, st>>>(ea, N, dc, t);
         prof_end((double)N * (8.0 * K + 16));
         prof_begin("pair_lone");
         pair_lone_kernel<K><<<grid_for(N, 1024, 8), 256, 0, st>>>(ea, N, dc, t);
@@ -3373,7 +3426,7 @@ static void run_group(State& s, const GroupSpec& gs) {
             ea.nbits = 1;
             ea.sqrt2inv = 1.0 / std::sqrt(2.0);
             ea.eps = gs.eps;
-            ea.sign2pi = gs.sign * 2 * 3.14159265358979323846;
+            ea.turn_neg = gs.sign < 0;
             for (int i = 0; i < 4; ++i) ea.m[i] = gs.m[i];
             ea.mtable = gs.mtable;
             ea.real = real_matrix(gs);
@@ -3471,7 +3524,7 @@ static void run_group(State& s, const GroupSpec& gs) {
     ea.extra = gs.unscaled ? 1.0 : 1.0 / std::sqrt((double)(1ull << gs.target.width));
     ea.sqrt2inv = 1.0 / std::sqrt(2.0);
     ea.eps = gs.eps;
-    ea.sign2pi = gs.sign * 2 * 3.14159265358979323846;
+    ea.turn_neg = gs.sign < 0;
     for (int i = 0; i < 4; ++i) ea.m[i] = gs.m[i];
     ea.mtable = gs.mtable;
     ea.real = real_matrix(gs);

@@ -1,10 +1,11 @@
 """1-bit splits by partner lookup at the sizes where their paths change: one
-CTA in shared memory up to 4096 entries, the claim table above it; target bits
+CTA in shared memory up to 2048 entries, the claim table above it; target bits
 that are constant (no partners), partly and fully paired; entries failing the
 conditions; every pair operator, one and several key words."""
 from __future__ import annotations
 
 import math
+from decimal import Decimal, localcontext
 
 import numpy as np
 import pytest
@@ -14,7 +15,7 @@ import sparqsim_gb300 as ps
 pytestmark = pytest.mark.gpu
 
 U = ps.UnsignedInteger
-SIZES = [1, 2, 255, 256, 257, 1024, 1025, 4096, 4097, 8193, 70001]
+SIZES = [1, 2, 255, 256, 257, 1025, 2048, 2049, 8193, 65536, 70001]
 
 
 def _rows(rng, n, bits, fill):
@@ -54,7 +55,7 @@ def test_pair_split_paths(dual, n, fill):
     dual.compare(exact_amp=True)
 
 
-@pytest.mark.parametrize("n", [5, 4096, 4097, 20000])
+@pytest.mark.parametrize("n", [5, 2048, 2049, 40000])
 @pytest.mark.parametrize("words", [1, 4, 8])
 def test_pair_split_key_words(dual, n, words):
     rng = np.random.default_rng(n + words)
@@ -71,6 +72,52 @@ def test_pair_split_key_words(dual, n, words):
     dual.compare(rel=1e-12)  # device sin/cos
     dual.apply(ps.Hadamard_Bool("q").conditioned_by_nonzeros("x"))
     dual.compare(rel=1e-12)
+
+
+def _cos_sin(v, w):
+    """cos and sin of 2 pi v / 2^w, from the Taylor series in 60 digits."""
+    with localcontext() as ctx:
+        ctx.prec = 60
+        pi = Decimal("3.14159265358979323846264338327950288419716939937510582097494459230781640628620899")
+        x = 2 * pi * Decimal(v) / Decimal(1 << w)
+        if x > pi:
+            x -= 2 * pi
+        s, c, t = Decimal(0), Decimal(0), Decimal(1)
+        for k in range(0, 80, 2):
+            c += t
+            t = t * x / (k + 1)
+            s += t
+            t = -t * x / (k + 2)
+        return c, s
+
+
+@pytest.mark.parametrize("w", [1, 2, 3, 7, 32, 53, 63, 64])
+def test_condrot_angles_are_correctly_rounded_to_an_ulp(w):
+    """Rotations of a lone |0> give (cos, sin): within 2^-52 relative of the
+    exact turn fraction (one rounding, 2^-53, and the series' 2^-61), also next
+    to the zeros, where entries below the prune threshold are dropped."""
+    rng = np.random.default_rng(w)
+    vals = {int(rng.integers(0, 1 << 62)) * 4 + 3 >> (64 - w) for _ in range(300)} | {0}
+    for e in range(8):  # the eighths of a turn and their neighbours
+        for d in (-2, -1, 0, 1, 2):
+            vals.add(((e << w) // 8 + d) % (1 << w))
+    ps.System.add_register("x", ps.Rational, w)
+    ps.System.add_register("q", ps.Boolean, 1)
+    for dag in (False, True):
+        st = ps.SparseState()
+        st.upload(np.array([[v, 0] for v in sorted(vals)], dtype=np.uint64), np.ones(len(vals), dtype=np.complex128))
+        op = ps.CondRot_Rational_Bool("x", "q")
+        (op.dag if dag else op)(st)
+        got = {(int(r[0]), int(r[1])): a for r, a in zip(*st.download())}
+        for v in vals:
+            for bit, e in enumerate(_cos_sin(v, w)):
+                if bit and dag:
+                    e = -e
+                a = got.get((v, bit))
+                if a is None:
+                    assert abs(e) < Decimal("1.0001e-7")
+                else:
+                    assert a.imag == 0 and abs(Decimal(float(a.real)) - e) <= abs(e) * Decimal(2) ** -52
 
 
 def test_small_split_in_a_graph():
