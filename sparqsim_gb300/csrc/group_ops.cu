@@ -1939,6 +1939,360 @@ __global__ void __launch_bounds__(512, 2) emit_h4096x_kernel(const __grid_consta
     ticket_exit(a.ticket);
 }
 
+// ------------------------------------------------------------------ tiles of 256 slots
+// Single-pass Hadamard_Int on up to 8 bits (or a batched width) in the
+// exact-sum arithmetic: a warp transforms 256 slots at a time, the slots of
+// one 8-bit group or of 2^(8 - n) groups of n bits, 8 slots per thread in
+// registers. Three slot bits at a time sit in the thread's index j: bits 5-7
+// (slot = j << 5 | lane, the layout the members are loaded in, coalesced),
+// bits 0-2 (lane << 3 | j) and bits 3-5 (lane_hi << 6 | j << 3 | lane_lo), with
+// two conflict-free shared-memory transposes between (swz8). A CTA takes a
+// chunk of groups, sorts them by width so that every tile is of one width and
+// as full as can be, and its warps take tiles from a counter.
+//
+// Merges leave few outputs, and a reservation per group costs 0.7 ns (400,000
+// of them, 0.3 ms, per merge of 4096 batched instances): outputs of tiles with
+// fewer than 32 wait in a queue of the warp and are reserved together.
+//
+// The warp-per-group kernel (emit_hadamard_kernel) keeps the slots in shared
+// memory: two reads and two writes per butterfly, half of the lanes idle on 16
+// members. The merges of 4096 batched instances of 4 to 8 bits (71 M entries
+// each): 733 us there, 496 here, now bound by integer issue (the ALU pipe 64 %
+// busy; about 2000 instructions per tile, of which 340 convert to the grid and
+// 256 are the butterflies). Also measured: rows unrolled (instruction cache
+// misses, 970 us), 3 CTAs of 8 warps at 80 registers (530 us), a copy for 8-bit
+// tiles with the width known to the compiler (508 us).
+constexpr unsigned kTileWarps = 4;    // per CTA
+constexpr unsigned kTileCtas = 4;     // per SM: 128 registers; at 80 the spills cost more than the warps gain
+constexpr unsigned kTileChunk = 128;  // groups per chunk at most
+constexpr unsigned kTileQueue = 64;   // waiting outputs per warp
+struct TileWarp {
+    double2 slot[256];
+    double2 qa[kTileQueue];
+    unsigned qhead[kTileQueue];  // an entry with the output's key
+    unsigned qslot[kTileQueue];  // target value | width << 16
+    unsigned qg[kTileQueue];     // groups of the waiting outputs: id, outputs | first << 16
+    unsigned qr[kTileQueue];
+    unsigned keep[8], before[8];  // per 32 slots: which are kept, outputs before them
+    unsigned short e[256];        // the tile's groups: largest exponent
+};
+struct TileCta {
+    TileWarp w[kTileWarps];
+    unsigned s0[kTileChunk], m[kTileChunk], head[kTileChunk], g[kTileChunk];  // sorted by width
+    unsigned cnt[9], start[9], partial[9], tiles[10], next;  // per width
+    unsigned long long ticket[2];
+};
+
+// x on the grid 2^(E - F), F = 62 - n for n <= 9 (to_fixed, without
+// branches): the mantissa moved up by 9 - n (up1 = 10 - n leaves one more bit
+// to round with), shifted right, rounded half away from zero.
+__device__ __forceinline__ long long to_fixed_small(double x, int emax, int up1) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const int ex = (int)(b >> 52) & 0x7ff;
+    const unsigned long long mant = ((b & 0xfffffffffffffull) | (ex ? (1ull << 52) : 0ull)) << up1;
+    const unsigned long long q = ((mant >> min(emax - max(ex, 1), 63)) + 1ull) >> 1;
+    const unsigned long long sg = 0ull - (b >> 63);
+    return (long long)((q ^ sg) - sg);
+}
+
+__device__ __forceinline__ void fwht_bit(longlong2 (&x)[8], int b) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        if (j & (1 << b)) continue;
+        const longlong2 x0 = x[j], x1 = x[j | (1 << b)];
+        x[j] = ladd(x0, x1);
+        x[j | (1 << b)] = lsub(x0, x1);
+    }
+}
+
+// Writes the warp's waiting outputs behind one reservation.
+template <int K>
+__device__ __forceinline__ void tile_flush(const EmitArgs& a, TileWarp& w, unsigned& nq, unsigned& ngq) {
+    const unsigned lane = threadIdx.x & 31u;
+    __syncwarp();
+    unsigned long long base = 0;
+    if (lane == 0 && nq) base = atomicAdd(a.cursor, (unsigned long long)nq);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (base + nq <= a.capacity) {
+        for (unsigned i = lane; i < nq; i += 32u) {
+            uint64_t k[K];
+            load_key<K>(a.in_keys, w.qhead[i], k);
+            Field tg = a.target;
+            tg.width = (uint8_t)(w.qslot[i] >> 16);
+            fset<K>(k, tg, (uint64_t)(w.qslot[i] & 0xffffu));
+            store_out<K>(a, base + i, k, w.qa[i]);
+        }
+    }
+    for (unsigned i = lane; a.ocnt && i < ngq; i += 32u) {
+        a.ostart[w.qg[i]] = base + (w.qr[i] >> 16);
+        a.ocnt[w.qg[i]] = w.qr[i] & 0xffffu;
+    }
+    __syncwarp();
+    nq = ngq = 0;
+}
+
+template <int K, int AM>
+__global__ void __launch_bounds__(32 * kTileWarps, kTileCtas) emit_tile_kernel(const __grid_constant__ EmitArgs a, unsigned chunk) {
+    extern __shared__ __align__(16) unsigned char s_tile_raw[];
+    TileCta& C = *reinterpret_cast<TileCta*>(s_tile_raw);
+    const unsigned tid = threadIdx.x, lane = tid & 31u;
+    TileWarp& w = C.w[tid >> 5];
+    const uint64_t groups = a.glist ? (uint64_t)*a.glist_n : a.groups;
+    const uint64_t chunks = (groups + chunk - 1) / chunk;
+    unsigned nq = 0, ngq = 0;
+    unsigned it = 0;
+    for (uint64_t ck = ticket_first(a.ticket, C.ticket); ck < chunks; ck = ticket_next(C.ticket, it)) {
+        ticket_prefetch(a.ticket, C.ticket, it);
+        // the chunk's groups, sorted by width; emptied cached ranges leave here
+        if (tid < 9u) {
+            C.cnt[tid] = 0u;
+            C.partial[tid] = 0u;
+        }
+        if (tid == 0) C.next = 0u;
+        __syncthreads();
+        const uint64_t gi = ck * chunk + tid;
+        unsigned g = 0, s0 = 0, m = 0, head = 0, pos = 0;
+        int n = 0;
+        if (tid < chunk && gi < groups) {
+            g = a.glist ? a.glist[gi] : (unsigned)gi;
+            group_range<AM>(a, g, s0, m);
+            if (m) {
+                head = group_head<AM>(a, g, s0);
+                n = a.nbits;
+                if (a.varw.width) n = (int)((a.in_keys.w[a.varw.word][head] >> a.varw.shift) & wmask(a.varw.width));
+                n = min(n, 8);  // the grouping refuses wider ones
+                pos = atomicAdd(&C.cnt[n], 1u);
+                if (AM != 2 || m != (1u << n) || m == 1u) C.partial[n] = 1u;
+            } else if (a.ocnt) {
+                a.ostart[g] = 0ull;
+                a.ocnt[g] = 0u;
+            }
+        }
+        __syncthreads();
+        if (tid == 0) {
+            unsigned st = 0, ti = 0;
+            for (int i = 0; i < 9; ++i) {
+                C.start[i] = st;
+                C.tiles[i] = ti;
+                st += C.cnt[i];
+                ti += (C.cnt[i] + (256u >> i) - 1u) >> (8 - i);
+            }
+            C.tiles[9] = ti;
+        }
+        __syncthreads();
+        if (m) {
+            const unsigned at = C.start[n] + pos;
+            C.s0[at] = s0;
+            C.m[at] = m;
+            C.head[at] = head;
+            C.g[at] = g;
+        }
+        __syncthreads();
+        const unsigned ntiles = C.tiles[9];
+        while (true) {
+            unsigned tile = 0;
+            if (lane == 0) tile = atomicAdd(&C.next, 1u);
+            tile = __shfl_sync(0xffffffffu, tile, 0);
+            if (tile >= ntiles) break;
+            // the tile's width: how many widths end at or before it
+            const int nb = __popc(__ballot_sync(0xffffffffu, lane < 8u && tile >= C.tiles[lane + 1u]));
+            const unsigned S = 1u << nb, per = 256u >> nb;
+            const unsigned first = C.start[nb] + (tile - C.tiles[nb]) * per;
+            const unsigned ng = min(per, C.start[nb] + C.cnt[nb] - first);
+            const bool direct = AM == 2 && !C.partial[nb];  // full cached ranges: member c has target c
+            longlong2 x[8];
+            {
+                int er[8];
+                double2 d[8];
+                if (direct) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const unsigned p = ((unsigned)j << 5) | lane, sub = p >> nb;
+                        d[j] = sub < ng ? __ldcs(a.in_amp + (C.s0[first + sub] + (p & (S - 1u)))) : make_double2(0.0, 0.0);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) er[j] = amp_exp(d[j]);
+                } else {
+                    unsigned t[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const unsigned p = ((unsigned)j << 5) | lane, sub = p >> nb, r = p & (S - 1u);
+                        const unsigned mm = sub < ng ? C.m[first + sub] : 0u;
+                        er[j] = 1;
+                        t[j] = 0xffffffffu;
+                        // a lone member is not transformed: written from its amplitude below
+                        if (r < mm && mm != 1u) {
+                            uint64_t tt;
+                            member_at<AM>(a, C.s0[first + sub] + r, tt, d[j]);
+                            t[j] = (sub << nb) | ((unsigned)tt & (S - 1u));
+                            er[j] = amp_exp(d[j]);
+                        }
+                        w.slot[p] = make_double2(0.0, 0.0);
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (t[j] != 0xffffffffu) w.slot[t[j]] = d[j];
+                    __syncwarp();
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) d[j] = w.slot[((unsigned)j << 5) | lane];
+                    __syncwarp();
+                }
+                // the largest exponent of each group
+                if (nb >= 5) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) er[j] = (int)__reduce_max_sync(0xffffffffu, (unsigned)er[j]);
+#pragma unroll
+                    for (int b = 0; b < 3; ++b) {
+                        if (nb <= 5 + b) break;
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            if (j & (1 << b)) continue;
+                            er[j] = er[j | (1 << b)] = max(er[j], er[j | (1 << b)]);
+                        }
+                    }
+                } else {
+                    for (int b = 0; b < nb; ++b) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) er[j] = max(er[j], __shfl_xor_sync(0xffffffffu, er[j], 1 << b));
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const unsigned p = ((unsigned)j << 5) | lane;
+                    if ((p & (S - 1u)) == 0u) w.e[p >> nb] = (unsigned short)er[j];
+                }
+                const int up1 = 10 - nb;
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    x[j] = make_longlong2(to_fixed_small(d[j].x, er[j], up1), to_fixed_small(d[j].y, er[j], up1));
+            }
+            if (nb > 5) fwht_bit(x, 0);
+            if (nb > 6) fwht_bit(x, 1);
+            if (nb > 7) fwht_bit(x, 2);
+            longlong2* ls = reinterpret_cast<longlong2*>(w.slot);
+            const unsigned c0 = ((lane >> 3) << 6) | (lane & 7u);
+#pragma unroll
+            for (unsigned j = 0; j < 8; ++j) ls[swz8((j << 5) | lane)] = x[j];
+            __syncwarp();
+#pragma unroll
+            for (unsigned j = 0; j < 8; ++j) x[j] = ls[swz8((lane << 3) | j)];
+            if (nb > 0) fwht_bit(x, 0);
+            if (nb > 1) fwht_bit(x, 1);
+            if (nb > 2) fwht_bit(x, 2);
+#pragma unroll
+            for (unsigned j = 0; j < 8; ++j) ls[swz8((lane << 3) | j)] = x[j];
+            __syncwarp();
+#pragma unroll
+            for (unsigned j = 0; j < 8; ++j) x[j] = ls[swz8(c0 | (j << 3))];
+            if (nb > 3) fwht_bit(x, 0);
+            if (nb > 4) fwht_bit(x, 1);
+#pragma unroll
+            for (unsigned j = 0; j < 8; ++j) ls[swz8(c0 | (j << 3))] = x[j];
+            __syncwarp();
+            // rows of 32 slots, in a loop (unrolled, the conversion and the
+            // output code overflowed the instruction cache). Merges leave most
+            // slots exactly zero: such rows are skipped.
+            unsigned total = 0, live = 0;
+#pragma unroll 1
+            for (unsigned r = 0; r < 8u; ++r) {
+                const unsigned c = (r << 5) | lane, sub = c >> nb;
+                const longlong2 y = ls[swz8(c)];
+                const bool lone = !direct && sub < ng && C.m[first + sub] == 1u;
+                unsigned ball = 0;
+                if (__any_sync(0xffffffffu, lone || (y.x | y.y) != 0)) {
+                    double2 v;
+                    bool keep;
+                    if (lone) {
+                        // singleton: a * 2^{-n/2}, sign (-1)^{popcount(t & v)} (hadamard.cpp:27-42)
+                        uint64_t v0;
+                        double2 a0;
+                        member_at<AM>(a, C.s0[first + sub], v0, a0);
+                        const double2 base = cscale(a0, a.varw.width ? inv_sqrt_pow2(nb, a.sqrt2inv) : a.extra);
+                        const bool neg = __popcll((uint64_t)(c & (S - 1u)) & v0) & 1;
+                        const long long sg = neg ? (long long)0x8000000000000000ull : 0ll;
+                        v = make_double2(__longlong_as_double(__double_as_longlong(base.x) ^ sg),
+                                         __longlong_as_double(__double_as_longlong(base.y) ^ sg));
+                        // batched width 0: the entry is left as it is, never pruned
+                        keep = (a.varw.width && nb == 0) || keep_amp(base, a.eps);
+                    } else {
+                        v = from_fixed2(y, fix_out_exp((int)w.e[sub], nb), nb & 1, a.sqrt2inv);
+                        keep = sub < ng && keep_amp(v, a.eps);
+                    }
+                    ball = __ballot_sync(0xffffffffu, keep);
+                    if (keep) ls[swz8(c)] = make_longlong2(__double_as_longlong(v.x), __double_as_longlong(v.y));
+                    live |= ball ? 1u << r : 0u;
+                }
+                if (lane == 0) {
+                    w.keep[r] = ball;
+                    w.before[r] = total;
+                }
+                total += __popc(ball);
+            }
+            __syncwarp();
+            const bool queued = total < 32u;
+            if (queued && (nq + total > kTileQueue || ngq + total > kTileQueue)) tile_flush<K>(a, w, nq, ngq);
+            unsigned long long base = 0;
+            bool fits = true;
+            if (!queued) {
+                if (lane == 0) base = atomicAdd(a.cursor, (unsigned long long)total);
+                base = __shfl_sync(0xffffffffu, base, 0);
+                fits = base + total <= a.capacity;
+            }
+            for (unsigned rr = fits ? live : 0u; rr; rr &= rr - 1u) {
+                const unsigned r = (unsigned)__ffs(rr) - 1u, ball = w.keep[r];
+                if (!((ball >> lane) & 1u)) continue;
+                const unsigned c = (r << 5) | lane, sub = c >> nb;
+                const unsigned rank = w.before[r] + __popc(ball & ((1u << lane) - 1u));
+                const longlong2 y = ls[swz8(c)];
+                const double2 v = make_double2(__longlong_as_double(y.x), __longlong_as_double(y.y));
+                const unsigned h = C.head[first + sub];
+                if (queued) {
+                    w.qa[nq + rank] = v;
+                    w.qhead[nq + rank] = h;
+                    w.qslot[nq + rank] = (c & (S - 1u)) | ((unsigned)nb << 16);
+                } else {
+                    uint64_t k[K];
+                    load_key<K>(a.in_keys, h, k);
+                    Field tg = a.target;
+                    tg.width = (uint8_t)nb;
+                    fset<K>(k, tg, (uint64_t)(c & (S - 1u)));
+                    store_out<K>(a, base + rank, k, v);
+                }
+            }
+            // the groups' output ranges, for the next split: outputs before a
+            // slot are those of the rows before it and of the row up to it
+            if (a.ocnt) {
+                for (unsigned b = 0; b < ng; b += 32u) {
+                    const unsigned sub = b + lane;
+                    unsigned cnt = 0, lo = 0;
+                    if (sub < ng) {
+                        const unsigned c = sub << nb, e = c + S;
+                        lo = w.before[c >> 5] + __popc(w.keep[c >> 5] & ((1u << (c & 31u)) - 1u));
+                        const unsigned hi = e >= 256u ? total : w.before[e >> 5] + __popc(w.keep[e >> 5] & ((1u << (e & 31u)) - 1u));
+                        cnt = hi - lo;
+                        if (!cnt || !queued) {
+                            a.ostart[C.g[first + sub]] = cnt ? base + lo : 0ull;
+                            a.ocnt[C.g[first + sub]] = cnt;
+                        }
+                    }
+                    const unsigned some = __ballot_sync(0xffffffffu, queued && cnt);
+                    if (queued && cnt) {
+                        const unsigned at = ngq + __popc(some & ((1u << lane) - 1u));
+                        w.qg[at] = C.g[first + sub];
+                        w.qr[at] = cnt | ((nq + lo) << 16);
+                    }
+                    ngq += __popc(some);
+                }
+            }
+            if (queued) nq += total;
+            __syncwarp();
+        }
+    }
+    tile_flush<K>(a, w, nq, ngq);
+    ticket_exit(a.ticket);
+}
+
 // Entries that fail the control conditions: copied through unchanged.
 template <int K>
 __global__ void passthrough_kernel(ConstKeyPtrs ik, const double2* __restrict__ ia, const unsigned* __restrict__ idx,
@@ -3341,6 +3695,25 @@ static void launch_hadamard(int am, unsigned grid, size_t sm, cudaStream_t st, c
     else if (am == 1) emit_hadamard_kernel<K, W, WRITE, 1><<<grid, 256, sm, st>>>(ea);
     else emit_hadamard_kernel<K, W, WRITE, 0><<<grid, 256, sm, st>>>(ea);
 }
+template <int K>
+static void launch_tile(int am, uint64_t G, cudaStream_t st, const EmitArgs& ea) {
+    static bool smem_set = false;
+    if (!smem_set) {
+        SQ_CUDA(cudaFuncSetAttribute(emit_tile_kernel<K, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileCta)));
+        SQ_CUDA(cudaFuncSetAttribute(emit_tile_kernel<K, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileCta)));
+        SQ_CUDA(cudaFuncSetAttribute(emit_tile_kernel<K, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileCta)));
+        smem_set = true;
+    }
+    // chunks of up to kTileChunk groups, smaller when the SMs would not all get a few
+    // (a fan-out's list of leftovers is short as a rule, its length unknown here)
+    const uint64_t want = ea.glist ? 8 : G / ((uint64_t)num_sms() * 8);
+    const unsigned chunk = (unsigned)std::min<uint64_t>(kTileChunk, std::max<uint64_t>(want, 8));
+    const unsigned grid = (unsigned)std::min<uint64_t>((G + chunk - 1) / chunk, (uint64_t)num_sms() * kTileCtas);
+    constexpr unsigned threads = 32 * kTileWarps;
+    if (am == 2) emit_tile_kernel<K, 2><<<grid, threads, sizeof(TileCta), st>>>(ea, chunk);
+    else if (am == 1) emit_tile_kernel<K, 1><<<grid, threads, sizeof(TileCta), st>>>(ea, chunk);
+    else emit_tile_kernel<K, 0><<<grid, threads, sizeof(TileCta), st>>>(ea, chunk);
+}
 template <int K, int NB, bool WRITE, bool UNI>
 static void launch_small_am(int am, unsigned grid, cudaStream_t st, const EmitArgs& ea) {
     if (am == 2) emit_small_kernel<K, NB, WRITE, 2, UNI><<<grid, 256, 0, st>>>(ea);
@@ -3667,6 +4040,8 @@ static void run_group(State& s, const GroupSpec& gs) {
                        : 2 * G <= P    ? "emit_hadamard_merge"
                                        : "emit_hadamard_single_pass");
             const unsigned fgrid = (unsigned)std::min<uint64_t>((G + 7) / 8, (uint64_t)num_sms() * 8);
+            const bool tiled = W == 32 && gs.mode == GM_HADAMARD_INT && ea.fix;
+            if (tiled) ea.ticket = group_ticket(st);
             if (fanout) {
                 ea.err = device_error_word();
                 // 256 groups per CTA and round (a group per lane)
@@ -3681,10 +4056,12 @@ static void run_group(State& s, const GroupSpec& gs) {
                 else emit_fanout_kernel<K, 0><<<ogrid, 256, 0, st>>>(ea);
                 if (G < P) {
                     SQ_CUDA(cudaGetLastError());
-                    launch_hadamard<K, 32, true>(am, fgrid, smem, st, ea);
+                    if (tiled) launch_tile<K>(am, G, st, ea);
+                    else launch_hadamard<K, 32, true>(am, fgrid, smem, st, ea);
                     ea.glist = ea.glist_n = nullptr;
                 }
-            } else if (W == 32) launch_hadamard<K, 32, true>(am, fgrid, smem, st, ea);
+            } else if (tiled) launch_tile<K>(am, G, st, ea);
+            else if (W == 32) launch_hadamard<K, 32, true>(am, fgrid, smem, st, ea);
             else launch_hadamard<K, 256, true>(am, (unsigned)std::min<uint64_t>(G, (uint64_t)num_sms() * 2), smem, st, ea);
             prof_end((double)P * E);
             SQ_CUDA(cudaGetLastError());
