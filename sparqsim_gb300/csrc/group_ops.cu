@@ -2306,42 +2306,56 @@ __global__ void passthrough_kernel(ConstKeyPtrs ik, const double2* __restrict__ 
     }
 }
 
-// ------------------------------------------------------------------ hash grouping
-// Group by an open-addressing hash table keyed on the masked group key. A slot
-// holds 0 (empty), kSlotLocked (being claimed) or ((gid + 1) << 32 | head + 1)
-// where `head` is the first entry that claimed it; keys are compared against
-// the head entry's key words. Group ids are dense, in claim order. Every wait
-// on a locked slot is bounded.
-constexpr unsigned long long kSlotLocked = ~0ull;
-
-// atomicAdd(ctr, 1) for each calling lane, one atomic per group of lanes that
-// execute the call together (new group ids: every lane of a warp of
-// singleton groups would otherwise hit the same counter)
-__device__ __forceinline__ unsigned warp_aggregated_add(unsigned* ctr) {
-    const unsigned am = __activemask();
-    const unsigned lane = threadIdx.x & 31u;
-    const int leader = __ffs(am) - 1;
-    unsigned base = 0;
-    if ((int)lane == leader) base = atomicAdd(ctr, (unsigned)__popc(am));
-    base = __shfl_sync(am, base, leader);
-    return base + (unsigned)__popc(am & ((1u << lane) - 1u));
+// Exclusive scan of a count over a CTA in thread order; `total` over the CTA.
+// s: one word per warp. Two barriers, so that s may be reused right away.
+template <int BLOCK>
+__device__ __forceinline__ unsigned block_rank(unsigned c, unsigned* s, unsigned& total) {
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    unsigned inc = c;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const unsigned v = __shfl_up_sync(0xffffffffu, inc, d);
+        if (lane >= (unsigned)d) inc += v;
+    }
+    if (lane == 31u) s[warp] = inc;
+    __syncthreads();
+    unsigned pre = 0, tot = 0;
+#pragma unroll
+    for (int w = 0; w < BLOCK / 32; ++w) {
+        const unsigned v = s[w];
+        if ((unsigned)w < warp) pre += v;
+        tot += v;
+    }
+    __syncthreads();
+    total = tot;
+    return pre + inc - c;
 }
 
+// ------------------------------------------------------------------ hash grouping
+// Group by an open-addressing hash table keyed on the masked group key. A slot
+// holds 0 (empty) or (fingerprint 24 | head + 1), `head` being the entry that
+// claimed it with one compare-and-swap; later entries of equal fingerprint
+// compare their masked key with the head's. The slot is the group's name while
+// members are counted; a scan over the slots then gives dense group numbers,
+// group starts and heads in one pass. Nothing waits on another thread.
+//
+// An earlier form numbered the groups from a global counter at each claim and
+// read the overflow flag at each probe: both are accesses of every lane to one
+// address (0.7 ns each) and made it the longest kernel of a CKS term (2.6 M
+// entries of 6 key words: 400 us a launch, 111 in this form; 400,000 entries of
+// one word, nearly all groups of one: 127 and 28).
 struct HashWs {
     unsigned long long* slots;
     unsigned long long cap_mask;
     unsigned* gcount;     // [0]: groups, [1]: entries failing the conditions, [2]: table overflow
-    unsigned* cnt;        // members per group
+    unsigned* cnt;        // per slot: members besides the head; after the scan: the group's next free position
     unsigned* head;       // one entry per group
-    unsigned* gid;        // group of each entry (~0u: fails the conditions)
+    unsigned* gid;        // slot of each entry (~0u: fails the conditions)
     unsigned* pass_list;  // entries failing the conditions
 };
 
-// The overflow flag is read coherently (another SM sets it while this lane
-// may be waiting on a slot that the setter locked and will never fill).
 __device__ __forceinline__ bool overflowed(const HashWs& h) {
-    cuda::atomic_ref<unsigned, cuda::thread_scope_device> f(h.gcount[2]);
-    return f.load(cuda::memory_order_relaxed) != 0u;
+    return *reinterpret_cast<volatile unsigned*>(h.gcount + 2) != 0u;
 }
 
 
@@ -2354,11 +2368,13 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
     return x;
 }
 
+// gmax: groups that the table may hold (half of its slots). More raise the
+// overflow flag, which ends the launch's remaining work; the host retries.
 template <int K>
 __global__ void __launch_bounds__(256) hash_insert_kernel(ConstKeyPtrs keys, const uint64_t* __restrict__ gmask,
                                                           DCondSet cond, uint64_t n, HashWs h, unsigned gmax,
                                                           Field tgt, Field varw, unsigned max_digits, unsigned* err) {
-    __shared__ unsigned s_fail[32];
+    __shared__ unsigned s_fail[8];
     __shared__ unsigned s_fail_base;
     uint64_t gm[K];
 #pragma unroll
@@ -2369,43 +2385,34 @@ __global__ void __launch_bounds__(256) hash_insert_kernel(ConstKeyPtrs keys, con
         const uint64_t i = b + threadIdx.x;
         const bool valid = i < n;
         uint64_t k[K];
-#pragma unroll
-        for (int w = 0; w < K; ++w) k[w] = valid ? (keys.w[w][i] & gm[w]) : 0ull;
         bool pass = false;
-        if (valid) {
+        {
             uint64_t full[K];
 #pragma unroll
-            for (int w = 0; w < K; ++w) full[w] = keys.w[w][i];
-            pass = cond_ok<K>(full, cond);
-            if (pass && varw.width) {  // batched Hadamard: drop this entry's own n low target bits
-                const unsigned nd = (unsigned)fget<K>(full, varw);
-                if (nd > max_digits) {
-                    atomicOr(err, 4u);
-                    pass = false;
-                } else {
-                    kword_set<K>(k, tgt.word, kword<K>(k, tgt.word) & ~(wmask(nd) << tgt.shift));
+            for (int w = 0; w < K; ++w) full[w] = valid ? keys.w[w][i] : 0ull;
+#pragma unroll
+            for (int w = 0; w < K; ++w) k[w] = full[w] & gm[w];
+            if (valid) {
+                pass = cond_ok<K>(full, cond);
+                if (pass && varw.width) {  // batched Hadamard: drop this entry's own n low target bits
+                    const unsigned nd = (unsigned)fget<K>(full, varw);
+                    if (nd > max_digits) {
+                        atomicOr(err, 4u);
+                        pass = false;
+                    } else {
+                        kword_set<K>(k, tgt.word, kword<K>(k, tgt.word) & ~(wmask(nd) << tgt.shift));
+                    }
                 }
+                if (!pass) h.gid[i] = ~0u;
             }
-            if (!pass) h.gid[i] = ~0u;
         }
-        {   // entries failing the conditions: one atomic per block and round
-            const bool fail = valid && !pass;
-            const unsigned fb = __ballot_sync(0xffffffffu, fail);
-            const unsigned warp = threadIdx.x >> 5;
-            if (lane == 0) s_fail[warp] = (unsigned)__popc(fb);
+        const bool fail = valid && !pass;
+        if (__syncthreads_or(fail)) {  // entries failing the conditions: one atomic per block and round
+            unsigned total;
+            const unsigned rank = block_rank<256>(fail ? 1u : 0u, s_fail, total);
+            if (threadIdx.x == 0) s_fail_base = atomicAdd(&h.gcount[1], total);
             __syncthreads();
-            if (threadIdx.x == 0) {
-                unsigned run = 0;
-                for (unsigned w = 0; w < (blockDim.x >> 5); ++w) {
-                    const unsigned c = s_fail[w];
-                    s_fail[w] = run;
-                    run += c;
-                }
-                s_fail_base = run ? atomicAdd(&h.gcount[1], run) : 0u;
-            }
-            __syncthreads();
-            if (fail) h.pass_list[s_fail_base + s_fail[warp] + __popc(fb & ((1u << lane) - 1u))] = (unsigned)i;
-            __syncthreads();
+            if (fail) h.pass_list[s_fail_base + rank] = (unsigned)i;
         }
         unsigned long long hv = 0x9e3779b97f4a7c15ull;
 #pragma unroll
@@ -2421,67 +2428,116 @@ __global__ void __launch_bounds__(256) hash_insert_kernel(ConstKeyPtrs keys, con
         for (int w = 0; w < K; ++w) same = same && (__shfl_sync(0xffffffffu, k[w], leader) == k[w]);
         const unsigned same_mask = __ballot_sync(0xffffffffu, pass && same);
         const bool probe = pass && (!same || (int)lane == leader);
-        unsigned mygid = ~0u;
+        unsigned myslot = ~0u;
+        bool claimed = false;
         if (probe) {
+            const unsigned long long tag = ((hv >> 40) << 32) | (unsigned long long)(i + 1);
             unsigned long long slot = hv & h.cap_mask;
-            unsigned spins = 0;
-            for (unsigned long long probes = 0; probes <= h.cap_mask;) {
-                if (overflowed(h)) break;  // table overflowed: the host retries with a larger one
-                cuda::atomic_ref<unsigned long long, cuda::thread_scope_device> ref(h.slots[slot]);
-                unsigned long long v = ref.load(cuda::memory_order_relaxed);
-                if (v == 0ull) {
-                    unsigned long long expected = 0ull;
-                    if (ref.compare_exchange_strong(expected, kSlotLocked, cuda::memory_order_relaxed)) {
-                        const unsigned g = warp_aggregated_add(&h.gcount[0]);
-                        if (g >= gmax) {
-                            atomicExch(&h.gcount[2], 1u);
-                            break;
-                        }
-                        h.head[g] = (unsigned)i;
-                        ref.store(((unsigned long long)(g + 1) << 32) | (unsigned long long)(i + 1),
-                                  cuda::memory_order_relaxed);
-                        mygid = g;
-                        break;
-                    }
-                    continue;  // lost the race: re-read this slot
-                }
-                if (v == kSlotLocked) {
-                    if (++spins > spin_limit(err)) {
-                        atomicOr(err, 2u);
-                        break;
-                    }
-                    __nanosleep(20);
-                    continue;
-                }
-                const unsigned hidx = (unsigned)(v & 0xffffffffull) - 1u;
-                uint64_t hk[K];
+            for (unsigned long long probes = 0; probes <= h.cap_mask; ++probes) {
+                const unsigned long long v = atomicCAS(&h.slots[slot], 0ull, tag);
+                claimed = v == 0ull;
+                bool eq = claimed;
+                if (!claimed && (v >> 32) == (tag >> 32)) {
+                    const unsigned hidx = (unsigned)(v & 0xffffffffull) - 1u;
+                    uint64_t hk[K];
 #pragma unroll
-                for (int w = 0; w < K; ++w) hk[w] = keys.w[w][hidx] & gm[w];
-                if (varw.width) {
-                    const unsigned hn = (unsigned)fget<K>(hk, varw);
-                    kword_set<K>(hk, tgt.word, kword<K>(hk, tgt.word) & ~(wmask(hn) << tgt.shift));
-                }
-                bool eq = true;
+                    for (int w = 0; w < K; ++w) hk[w] = __ldg(keys.w[w] + hidx) & gm[w];
+                    if (varw.width) {
+                        const unsigned hn = (unsigned)fget<K>(hk, varw);
+                        kword_set<K>(hk, tgt.word, kword<K>(hk, tgt.word) & ~(wmask(hn) << tgt.shift));
+                    }
+                    eq = true;
 #pragma unroll
-                for (int w = 0; w < K; ++w) eq = eq && ((hk[w] ^ k[w]) == 0);
+                    for (int w = 0; w < K; ++w) eq = eq && hk[w] == k[w];
+                }
                 if (eq) {
-                    mygid = (unsigned)(v >> 32) - 1u;
+                    myslot = (unsigned)slot;
                     break;
                 }
                 slot = (slot + 1) & h.cap_mask;
-                ++probes;
+                if ((probes & 31u) == 31u && overflowed(h)) break;
             }
-            if (mygid != ~0u) {
-                const unsigned c = (int)lane == leader ? __popc(peers & same_mask) : 1u;
-                atomicAdd(&h.cnt[mygid], c);
+            if (myslot != ~0u) {
+                const unsigned c = ((int)lane == leader ? __popc(peers & same_mask) : 1u) - (claimed ? 1u : 0u);
+                if (c) atomicAdd(&h.cnt[myslot], c);
+            } else {
+                h.gcount[2] = 1u;  // the table is full
             }
         }
-        const unsigned lg = __shfl_sync(0xffffffffu, mygid, leader);
-        if (pass) {
-            if (!probe) mygid = lg;
-            h.gid[i] = mygid;
-            if (mygid == ~0u && !overflowed(h)) atomicOr(err, 2u);  // probe gave up: reported
+        const unsigned lg = __shfl_sync(0xffffffffu, myslot, leader);
+        if (pass) h.gid[i] = probe ? myslot : lg;
+        const int claims = __syncthreads_count(claimed);
+        bool stop = false;
+        if (threadIdx.x == 0) {
+            if (claims && atomicAdd(&h.gcount[0], (unsigned)claims) + (unsigned)claims > gmax) h.gcount[2] = 1u;
+            stop = overflowed(h);
         }
+        if (__syncthreads_or(stop)) break;
+    }
+}
+
+// Dense groups from the table, in slot order: each occupied slot's group
+// number and first position come from one look-back scan of (groups, members)
+// packed into a word; the slot's count becomes its next free position.
+__global__ void __launch_bounds__(kSelBlock) slots_scan_kernel(HashWs h, unsigned* __restrict__ seg, LbWs lb,
+                                                               long long ntiles, unsigned* err) {
+    __shared__ unsigned s_tile;
+    __shared__ unsigned long long s_w[kSelBlock / 32];
+    __shared__ unsigned long long s_prefix;
+    if (overflowed(h)) return;
+    const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    if (tid == 0) s_tile = atomicAdd(lb.counter, 1u);
+    __syncthreads();
+    const long long tile = s_tile;
+    const uint64_t base = (uint64_t)tile * kSelTile + (uint64_t)tid * kSelItems;
+    unsigned head[kSelItems], cnt[kSelItems];
+    unsigned long long sum = 0;  // groups << 31 | members (both at most 2^30)
+#pragma unroll
+    for (int j = 0; j < kSelItems; j += 2) {
+        ulonglong2 v = make_ulonglong2(0ull, 0ull);
+        if (base + j <= h.cap_mask) v = *reinterpret_cast<const ulonglong2*>(h.slots + base + j);  // the capacity is even
+        head[j] = (unsigned)v.x;
+        head[j + 1] = (unsigned)v.y;
+    }
+#pragma unroll
+    for (int j = 0; j < kSelItems; ++j) {
+        cnt[j] = head[j] ? h.cnt[base + j] + 1u : 0u;
+        if (head[j]) sum += (1ull << 31) | cnt[j];
+    }
+    unsigned long long inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        unsigned long long t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= (unsigned)o) inc += t;
+    }
+    if (lane == 31) s_w[warp] = inc;
+    __syncthreads();
+    if (warp == 0) {
+        unsigned long long wv = lane < kSelBlock / 32 ? s_w[lane] : 0ull;
+        unsigned long long wi = wv;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            unsigned long long t = __shfl_up_sync(0xffffffffu, wi, o);
+            if (lane >= (unsigned)o) wi += t;
+        }
+        const unsigned long long total = __shfl_sync(0xffffffffu, wi, kSelBlock / 32 - 1);
+        if (lane < kSelBlock / 32) s_w[lane] = wi - wv;
+        unsigned long long pre = lb_warp_exclusive(lb.status, tile, total, err);
+        if (lane == 0) {
+            s_prefix = pre;
+            if (tile == ntiles - 1) seg[(pre + total) >> 31] = (unsigned)((pre + total) & 0x7fffffffull);  // the end
+        }
+    }
+    __syncthreads();
+    unsigned long long run = s_prefix + s_w[warp] + inc - sum;
+#pragma unroll
+    for (int j = 0; j < kSelItems; ++j) {
+        if (!head[j]) continue;
+        const unsigned g = (unsigned)(run >> 31), off = (unsigned)(run & 0x7fffffffull);
+        seg[g] = off;
+        h.head[g] = head[j] - 1u;
+        h.cnt[base + j] = off;
+        run += (1ull << 31) | cnt[j];
     }
 }
 
@@ -2729,86 +2785,32 @@ __global__ void __launch_bounds__(1024) group_small_kernel(const __grid_constant
 }
 
 // Partition the condition-passing entries by group: each entry's target value
-// and amplitude land in its group's range [seg[g], seg[g+1]); lanes of a warp
-// with the same group reserve consecutive slots with one atomic.
-__global__ void __launch_bounds__(256) bucket_kernel(const unsigned* __restrict__ gid, const uint64_t* __restrict__ tword,
-                                                     Field target, const double2* __restrict__ amp, uint64_t n,
-                                                     const unsigned* __restrict__ seg, unsigned* __restrict__ cnt,
+// and amplitude land in its group's range; lanes of a warp with the same group
+// reserve consecutive positions with one atomic.
+__global__ void __launch_bounds__(256) bucket_kernel(HashWs h, const uint64_t* __restrict__ tword, Field target,
+                                                     const double2* __restrict__ amp, uint64_t n,
                                                      unsigned* __restrict__ btgt, double2* __restrict__ bamp,
                                                      const uint64_t* __restrict__ wword, Field varw) {
+    if (overflowed(h)) return;
     const unsigned lane = threadIdx.x & 31u;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t base0 = (uint64_t)blockIdx.x * blockDim.x;
     for (uint64_t b = base0; b < n; b += stride) {  // warp-uniform trip count
         const uint64_t i = b + threadIdx.x;
-        const unsigned g = i < n ? gid[i] : ~0u;
+        const unsigned g = i < n ? h.gid[i] : ~0u;
         const bool valid = g != ~0u;
         const unsigned vmask = __ballot_sync(0xffffffffu, valid);
         const unsigned peers = __match_any_sync(0xffffffffu, g) & vmask;
         if (valid) {
             const int leader = __ffs(peers) - 1;
             const unsigned rank = __popc(peers & ((1u << lane) - 1u));
-            unsigned old = 0;
-            if ((int)lane == leader) old = atomicSub(&cnt[g], (unsigned)__popc(peers));
-            old = __shfl_sync(peers, old, leader);
-            const unsigned pos = seg[g] + old - 1u - rank;
+            unsigned pos = 0;
+            if ((int)lane == leader) pos = atomicAdd(&h.cnt[g], (unsigned)__popc(peers));
+            pos = __shfl_sync(peers, pos, leader) + rank;
             const unsigned nd = varw.width ? (unsigned)((wword[i] >> varw.shift) & wmask(varw.width)) : target.width;
             btgt[pos] = (unsigned)((tword[i] >> target.shift) & wmask(nd));
             bamp[pos] = amp[i];
         }
-    }
-}
-
-// Exclusive scan of u32 counts into u32 group starts (seg[G] is written by the host).
-__global__ void __launch_bounds__(kSelBlock) scan_seg_kernel(const unsigned* __restrict__ cnt, unsigned* __restrict__ seg,
-                                                             uint64_t n, LbWs lb, long long ntiles, unsigned* err) {
-    __shared__ unsigned s_tile;
-    __shared__ unsigned long long s_w[kSelBlock / 32];
-    __shared__ unsigned long long s_prefix;
-    const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    if (tid == 0) s_tile = atomicAdd(lb.counter, 1u);
-    __syncthreads();
-    const long long tile = s_tile;
-    const uint64_t base = (uint64_t)tile * kSelTile + (uint64_t)tid * kSelItems;
-    unsigned long long v[kSelItems];
-    unsigned long long sum = 0;
-#pragma unroll
-    for (int j = 0; j < kSelItems; ++j) {
-        const uint64_t i = base + j;
-        v[j] = i < n ? cnt[i] : 0ull;
-        sum += v[j];
-    }
-    unsigned long long inc = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        unsigned long long t = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= (unsigned)o) inc += t;
-    }
-    if (lane == 31) s_w[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-        unsigned long long wv = lane < kSelBlock / 32 ? s_w[lane] : 0ull;
-        unsigned long long wi = wv;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            unsigned long long t = __shfl_up_sync(0xffffffffu, wi, o);
-            if (lane >= (unsigned)o) wi += t;
-        }
-        const unsigned long long total = __shfl_sync(0xffffffffu, wi, kSelBlock / 32 - 1);
-        if (lane < kSelBlock / 32) s_w[lane] = wi - wv;
-        unsigned long long pre = lb_warp_exclusive(lb.status, tile, total, err);
-        if (lane == 0) {
-            s_prefix = pre;
-            if (tile == ntiles - 1) *lb.total = pre + total;
-        }
-    }
-    __syncthreads();
-    unsigned long long run = s_prefix + s_w[warp] + inc - sum;
-#pragma unroll
-    for (int j = 0; j < kSelItems; ++j) {
-        const uint64_t i = base + j;
-        if (i < n) seg[i] = (unsigned)run;
-        run += v[j];
     }
 }
 
@@ -3111,25 +3113,24 @@ static Grouping group_by_hash(State& s, const GroupSpec& gs, uint64_t* dg, uint6
         return out;
     }
     // Table sized for the expected number of groups (load factor <= 1/2);
-    // if more groups show up the kernel flags overflow and we retry with a
-    // table that fits every entry.
+    // if more groups show up the kernels flag overflow and we retry with a
+    // table that fits every entry. The scan and the bucket pass need no count
+    // on the host, so the whole grouping is read back once.
     uint64_t want = std::min<uint64_t>(N, want_groups ? want_groups : hash_groups_hint());
-    HashWs h;
-    char* base = nullptr;
-    size_t off_btgt = 0, off_bamp = 0;
-    for (int attempt = 0; attempt < 2; ++attempt) {
+    for (int attempt = 0;; ++attempt) {
         uint64_t cap = 1024;
         while (cap < 2 * want) cap <<= 1;
-        const uint64_t gmax = cap / 2;
+        const uint64_t most = std::min<uint64_t>(N, cap);  // groups that a full table can hold
         // one allocation: slots | counters | cnt | head | gid | pass_list | bucket target | bucket amp
         const size_t off_cnt = cap * 8 + 256;
-        const size_t off_head = off_cnt + gmax * 4;
-        const size_t off_gid = off_head + gmax * 4;
+        const size_t off_head = off_cnt + cap * 4;
+        const size_t off_gid = off_head + most * 4;
         const size_t off_pass = off_gid + N * 4;
-        off_btgt = off_pass + N * 4;
-        off_bamp = (off_btgt + N * 4 + 15) & ~size_t(15);
+        const size_t off_btgt = off_pass + N * 4;
+        const size_t off_bamp = (off_btgt + N * 4 + 15) & ~size_t(15);
         const size_t total = off_bamp + N * 16;
-        base = (char*)ws().get(WS_MERGE_KEYS, total);
+        char* base = (char*)ws().get(WS_MERGE_KEYS, total);
+        HashWs h;
         h.slots = (unsigned long long*)base;
         h.cap_mask = cap - 1;
         h.gcount = (unsigned*)(base + cap * 8);
@@ -3137,51 +3138,46 @@ static Grouping group_by_hash(State& s, const GroupSpec& gs, uint64_t* dg, uint6
         h.head = (unsigned*)(base + off_head);
         h.gid = (unsigned*)(base + off_gid);
         h.pass_list = (unsigned*)(base + off_pass);
+        unsigned* btgt = (unsigned*)(base + off_btgt);
+        double2* bamp = (double2*)(base + off_bamp);
+        unsigned* seg = (unsigned*)ws().get(WS_SEG, (most + 2) * 4);
         SQ_CUDA(cudaMemsetAsync(base, 0, off_head, st));  // slots, counters, cnt
         prof_begin("hash_insert");
-        hash_insert_kernel<K><<<grid_for(N, 256, 8), 256, 0, st>>>(ik, dg, gs.cond, N, h, (unsigned)gmax, gs.target,
+        hash_insert_kernel<K><<<grid_for(N, 256, 8), 256, 0, st>>>(ik, dg, gs.cond, N, h, (unsigned)(cap / 2), gs.target,
                                                                    gs.varw, gs.target.width, device_error_word());
         prof_end((double)N * (8.0 * K + 4));
+        SQ_CUDA(cudaGetLastError());
+        const long long nt = (long long)((cap + kSelTile - 1) / kSelTile);
+        LbWs lb = make_lb(nt);
+        prof_begin("scan_group_sizes");
+        slots_scan_kernel<<<(unsigned)nt, kSelBlock, 0, st>>>(h, seg, lb, nt, device_error_word());
+        prof_end((double)cap * 12);
+        SQ_CUDA(cudaGetLastError());
+        prof_begin("bucket_members");
+        bucket_kernel<<<grid_for(N, 256, 8), 256, 0, st>>>(h, s.live.keys[gs.target.word], gs.target, s.live.amp, N,
+                                                           btgt, bamp, s.live.keys[gs.varw.width ? gs.varw.word : 0],
+                                                           gs.varw);
+        prof_end((double)N * (4 + 8 + 16) + (double)N * (4 + 16 + 8));
         SQ_CUDA(cudaGetLastError());
         unsigned gc[3] = {0, 0, 0};
         host_read(gc, h.gcount, 12);
         check_device_error();
-        if (!gc[2]) break;
-        if (attempt == 1) fail(SQ_ERR_DEVICE_TIMEOUT, "hash grouping overflowed a table sized for every entry");
-        want = N;
-    }
-    unsigned gc[2] = {0, 0};
-    host_read(gc, h.gcount, 8);
-    Grouping out;
-    out.G = gc[0];
-    out.F = gc[1];
-    out.pass = h.pass_list;
-    out.ghead = h.head;
-    out.bucket = true;
-    const uint64_t P = N - out.F;
-    unsigned* seg = (unsigned*)ws().get(WS_SEG, (out.G + 2) * 4);
-    out.seg = seg;
-    if (out.G > 0) {
-        const long long nt = (long long)((out.G + kSelTile - 1) / kSelTile);
-        LbWs lb = make_lb(nt);
-        prof_begin("scan_group_sizes");
-        scan_seg_kernel<<<(unsigned)nt, kSelBlock, 0, st>>>(h.cnt, seg, out.G, lb, nt, device_error_word());
-        prof_end((double)out.G * 8);
-        SQ_CUDA(cudaGetLastError());
-        unsigned endv = (unsigned)P;
-        h2d_small(seg + out.G, &endv, 4);
-        unsigned* btgt = (unsigned*)(base + off_btgt);
-        double2* bamp = (double2*)(base + off_bamp);
-        prof_begin("bucket_members");
-        bucket_kernel<<<grid_for(N, 256, 8), 256, 0, st>>>(h.gid, s.live.keys[gs.target.word], gs.target, s.live.amp,
-                                                           N, seg, h.cnt, btgt, bamp,
-                                                           s.live.keys[gs.varw.width ? gs.varw.word : 0], gs.varw);
-        prof_end((double)N * (4 + 8 + 16) + (double)P * (4 + 16 + 8));
-        SQ_CUDA(cudaGetLastError());
+        if (gc[2]) {
+            if (attempt == 1) fail(SQ_ERR_DEVICE_TIMEOUT, "hash grouping overflowed a table sized for every entry");
+            want = N;
+            continue;
+        }
+        Grouping out;
+        out.G = gc[0];
+        out.F = gc[1];
+        out.seg = seg;
+        out.pass = h.pass_list;
+        out.ghead = h.head;
+        out.bucket = true;
         out.btgt = btgt;
         out.bamp = bamp;
+        return out;
     }
-    return out;
 }
 
 // ------------------------------------------------------------------ pair splits by partner lookup
@@ -3190,10 +3186,9 @@ static Grouping group_by_hash(State& s, const GroupSpec& gs, uint64_t* dg, uint6
 // an open-addressing table on the key without the target bit. The first to
 // arrive leaves its index in the slot; the second finds it there, knows both
 // members and writes the pair's outputs at once (pair_math, the arithmetic of
-// the grouped path). Entries that met nobody are written by a last pass, and
-// so are the entries that fail the conditions (copied). A slot is
-// (fingerprint 24 | index + 1), zero empty; the table holds at least twice the
-// entries, so every probe sequence ends at an empty slot.
+// the grouped path). Entries that met nobody are written by a last pass. A slot is
+// (fingerprint 24 | index + 1), zero empty; the table has more slots than
+// entries, so every probe sequence ends.
 //
 // What bounds it: the random table accesses (2^21 random 64-bit
 // compare-and-swaps take 40 us, as many random loads 15 us; at 2^24, where the
@@ -3230,31 +3225,6 @@ __device__ __forceinline__ bool is_partner(const ConstKeyPtrs& keys, unsigned lo
 #pragma unroll
     for (int w = 0; w < K; ++w) eq = eq && __ldg(keys.w[w] + j) == ((unsigned)w == tw ? k[w] ^ bit : k[w]);
     return eq;
-}
-
-// Exclusive scan of a count over a CTA in thread order; `total` over the CTA.
-// s: one word per warp. Two barriers, so that s may be reused right away.
-template <int BLOCK>
-__device__ __forceinline__ unsigned block_rank(unsigned c, unsigned* s, unsigned& total) {
-    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    unsigned inc = c;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const unsigned v = __shfl_up_sync(0xffffffffu, inc, d);
-        if (lane >= (unsigned)d) inc += v;
-    }
-    if (lane == 31u) s[warp] = inc;
-    __syncthreads();
-    unsigned pre = 0, tot = 0;
-#pragma unroll
-    for (int w = 0; w < BLOCK / 32; ++w) {
-        const unsigned v = s[w];
-        if ((unsigned)w < warp) pre += v;
-        tot += v;
-    }
-    __syncthreads();
-    total = tot;
-    return pre + inc - c;
 }
 
 // One reservation on the output cursor per CTA (a reservation per warp put
@@ -3373,7 +3343,7 @@ __global__ void __launch_bounds__(256) pair_claim_kernel(const __grid_constant__
 #pragma unroll
             for (int q = 0; q < ITEMS; ++q) {
                 if (!((pass >> q) & 1u)) continue;
-                // at most capacity probes; the table is at most half full
+                // at most capacity probes; the table is never full
                 for (unsigned long long probes = 0; v[q] != 0ull && probes <= t.mask; ++probes) {
                     if ((v[q] >> 32) == (tag[q] >> 32) &&
                         is_partner<K>(a.in_keys, (v[q] & 0xffffffffull) - 1ull, k[q], tw, bit)) {
@@ -3504,7 +3474,7 @@ __global__ void __launch_bounds__(BLOCK) pair_small_kernel(const __grid_constant
             continue;
         }
         unsigned slot = (unsigned)pair_hash<K>(k, tw, bit) & (cap - 1u);
-        for (unsigned probes = 0; probes < cap; ++probes) {  // at most half full: ends at an empty slot
+        for (unsigned probes = 0; probes < cap; ++probes) {  // never full: ends at an empty slot
             const unsigned old = atomicCAS(&table[slot], 0u, e + 1u);
             if (old == 0u) break;
             if (is_partner<K>(a.in_keys, old - 1u, k, tw, bit)) {
@@ -3574,8 +3544,9 @@ static void run_pair_partner(State& s, const GroupSpec& gs, EmitArgs& ea) {
     unsigned long long* cur = (unsigned long long*)ws().get(WS_CURSOR, 64);
     ea.cursor = cur;
     ea.capacity = capT;
+    // at most two thirds full if no entry had a partner (pairs share a slot)
     uint64_t cap = N <= kPairSmallMax ? 32 : 1024;
-    while (cap < 2 * N) cap <<= 1;
+    while (cap < N + N / 2) cap <<= 1;
     unsigned long long T = 0;
     if (N <= kPairSmallMax) {
         const MailSlot mail = mail_slot();
