@@ -23,7 +23,7 @@ struct DField {
     uint8_t shift;
     uint8_t width;
     uint8_t type;
-    uint32_t pad;
+    uint32_t mask32;  // low half of mask
     uint64_t mask;   // wmask(width)
     uint64_t smask;  // mask << shift
 };
@@ -33,25 +33,29 @@ static DField dfield(const Field& f) {
     d.shift = f.shift;
     d.width = f.width;
     d.type = f.type;
-    d.pad = 0;
     d.mask = wmask(f.width);
+    d.mask32 = (uint32_t)d.mask;
     d.smask = d.mask << f.shift;
     return d;
 }
+// The key words of an entry that a program uses.
 template <int K>
-__device__ __forceinline__ uint64_t fget(const uint64_t (&k)[K], const DField& f) {
-    return (kword<K>(k, f.word) >> f.shift) & f.mask;
+struct WordRegs {
+    uint64_t k[K];
+};
+template <int K>
+__device__ __forceinline__ uint64_t fget(const WordRegs<K>& r, const DField& f) {
+    return (kword<K>(r.k, f.word) >> f.shift) & f.mask;
 }
 template <int K>
-__device__ __forceinline__ void fset(uint64_t (&k)[K], const DField& f, uint64_t v) {
-    const uint64_t w = kword<K>(k, f.word);
-    kword_set<K>(k, f.word, (w & ~f.smask) | ((v << f.shift) & f.smask));
+__device__ __forceinline__ void fset(WordRegs<K>& r, const DField& f, uint64_t v) {
+    const uint64_t w = kword<K>(r.k, f.word);
+    kword_set<K>(r.k, f.word, (w & ~f.smask) | ((v << f.shift) & f.smask));
 }
-
 struct DInstr {
     uint16_t op;
     uint8_t dag;
-    uint8_t pad;
+    uint8_t narrow;  // may run in exec_narrow
     uint32_t addr_bits;
     uint64_t amask;  // wmask(addr_bits)
     DField f[4];
@@ -60,10 +64,18 @@ struct DInstr {
     const void* table;
     uint32_t elem_bytes;
     uint32_t pad2;
-    uint64_t zmask[SQ_KMAX];
+    uint64_t zmask[SQ_KMAX];  // reflections: the registers' bits per key word
     DCondSet cond;
 };
-
+template <int K>
+__device__ __forceinline__ bool holds(const WordRegs<K>& r, const DCondSet& cs) { return cond_ok<K>(r.k, cs); }
+template <int K>
+__device__ __forceinline__ bool all_zero(const WordRegs<K>& r, const uint64_t* zmask) {
+    bool z = true;
+#pragma unroll
+    for (int w = 0; w < K; ++w) z = z && ((r.k[w] & zmask[w]) == 0);
+    return z;
+}
 template <int MAXI>
 struct ProgramArgs {
     unsigned* err;         // device error word (bit 3: a lookup value without a table entry)
@@ -139,27 +151,41 @@ __device__ __forceinline__ uint64_t bits_deposit(uint64_t v, uint64_t m) {
     return out;
 }
 
-template <int K>
-__device__ __forceinline__ void exec(const DInstr& in, uint64_t (&k)[K], double2& a, unsigned* err) {
+// One instruction on the Q entries of a thread: the opcode is decoded once,
+// entries that fail its conditions are left out (ok).
+#define SQ_EACH(...)                              \
+    _Pragma("unroll") for (int q = 0; q < Q; ++q) { \
+        if (!ok[q]) continue;                     \
+        R& k = kk[q];                             \
+        double2& a = aa[q];                       \
+        (void)k;                                  \
+        (void)a;                                  \
+        __VA_ARGS__                               \
+    }
+template <typename R, int Q>
+__device__ __forceinline__ void exec(const DInstr& in, R (&kk)[Q], double2 (&aa)[Q], const bool (&ok)[Q],
+                                     unsigned* err) {
     const DField* f = in.f;
     switch (in.op) {
-        case SQ_OP_FLIP_BOOLS: fset<K>(k, f[0], ~fget<K>(k, f[0])); break;
-        case SQ_OP_SWAP_BOOL_BOOL: {
-            uint64_t x = fget<K>(k, f[0]), y = fget<K>(k, f[1]);
+        case SQ_OP_FLIP_BOOLS: SQ_EACH(fset(k, f[0], ~fget(k, f[0]));) break;
+        case SQ_OP_SWAP_BOOL_BOOL:
+            SQ_EACH({
+            uint64_t x = fget(k, f[0]), y = fget(k, f[1]);
             const uint64_t d1 = in.imm[0], d2 = in.imm[1];
             const bool v1 = (x >> d1) & 1, v2 = (y >> d2) & 1;
             if (v1 && !v2) { x -= 1ull << d1; y += 1ull << d2; }
             if (v2 && !v1) { x += 1ull << d1; y -= 1ull << d2; }
-            fset<K>(k, f[0], x);
-            fset<K>(k, f[1], y);
+            fset(k, f[0], x);
+            fset(k, f[1], y);
+            })
             break;
-        }
         case SQ_OP_SHIFT_LEFT:
-        case SQ_OP_SHIFT_RIGHT: {
+        case SQ_OP_SHIFT_RIGHT:
+            SQ_EACH({
             const unsigned size = f[0].width;
             const unsigned d = (unsigned)in.imm[0];
             const bool left = (in.op == SQ_OP_SHIFT_LEFT) != (in.dag != 0);
-            const uint64_t v = fget<K>(k, f[0]);
+            const uint64_t v = fget(k, f[0]);
             uint64_t r;
             if (left) {
                 const uint64_t high = shr(v, size - d);
@@ -170,149 +196,161 @@ __device__ __forceinline__ void exec(const DInstr& in, uint64_t (&k)[K], double2
                 const uint64_t low = v - shl(high, d);
                 r = shl(low, size - d) + high;
             }
-            fset<K>(k, f[0], r);
+            fset(k, f[0], r);
+            })
             break;
-        }
-        case SQ_OP_MULT_UINT_CONST: fset<K>(k, f[2], fget<K>(k, f[2]) ^ (fget<K>(k, f[0]) * in.imm[0])); break;
-        case SQ_OP_ADD_MULT_UINT_CONST: {
-            const uint64_t o = fget<K>(k, f[2]), l = fget<K>(k, f[0]);
-            fset<K>(k, f[2], in.dag ? o - l * in.imm[0] : o + in.imm[0] * l);
+        case SQ_OP_MULT_UINT_CONST: SQ_EACH(fset(k, f[2], fget(k, f[2]) ^ (fget(k, f[0]) * in.imm[0]));) break;
+        case SQ_OP_ADD_MULT_UINT_CONST:
+            SQ_EACH({
+            const uint64_t o = fget(k, f[2]), l = fget(k, f[0]);
+            fset(k, f[2], in.dag ? o - l * in.imm[0] : o + in.imm[0] * l);
+            })
             break;
-        }
-        case SQ_OP_MOD_MULT_CONST: fset<K>(k, f[0], (fget<K>(k, f[0]) * in.imm[0]) % in.imm[1]); break;
-        case SQ_OP_ADD_UINT_UINT: fset<K>(k, f[2], fget<K>(k, f[2]) ^ (fget<K>(k, f[0]) + fget<K>(k, f[1]))); break;
-        case SQ_OP_ADD_UINT_UINT_INPLACE: {
-            const uint64_t o = fget<K>(k, f[1]), l = fget<K>(k, f[0]);
-            fset<K>(k, f[1], in.dag ? o - l : o + l);
+        case SQ_OP_MOD_MULT_CONST: SQ_EACH(fset(k, f[0], (fget(k, f[0]) * in.imm[0]) % in.imm[1]);) break;
+        case SQ_OP_ADD_UINT_UINT: SQ_EACH(fset(k, f[2], fget(k, f[2]) ^ (fget(k, f[0]) + fget(k, f[1])));) break;
+        case SQ_OP_ADD_UINT_UINT_INPLACE:
+            SQ_EACH({
+            const uint64_t o = fget(k, f[1]), l = fget(k, f[0]);
+            fset(k, f[1], in.dag ? o - l : o + l);
+            })
             break;
-        }
-        case SQ_OP_ADD_UINT_CONST: fset<K>(k, f[2], fget<K>(k, f[2]) ^ (fget<K>(k, f[0]) + in.imm[0])); break;
-        case SQ_OP_ADD_CONST_INPLACE: {
-            const uint64_t o = fget<K>(k, f[0]);
-            fset<K>(k, f[0], in.dag ? o - in.imm[0] : o + in.imm[0]);
+        case SQ_OP_ADD_UINT_CONST: SQ_EACH(fset(k, f[2], fget(k, f[2]) ^ (fget(k, f[0]) + in.imm[0]));) break;
+        case SQ_OP_ADD_CONST_INPLACE:
+            SQ_EACH({
+            const uint64_t o = fget(k, f[0]);
+            fset(k, f[0], in.dag ? o - in.imm[0] : o + in.imm[0]);
+            })
             break;
-        }
-        case SQ_OP_PLUS_ONE_OVERFLOW: {
-            const uint64_t v = fget<K>(k, f[0]);
+        case SQ_OP_PLUS_ONE_OVERFLOW:
+            SQ_EACH({
+            const uint64_t v = fget(k, f[0]);
             const uint64_t top = wmask(f[0].width);
             const bool wrap = in.dag ? v == 0 : v == top;
-            fset<K>(k, f[0], in.dag ? v - 1 : v + 1);  // stored modulo 2^width
-            if (wrap) fset<K>(k, f[1], (fget<K>(k, f[1]) + 1) % 2);
+            fset(k, f[0], in.dag ? v - 1 : v + 1);  // stored modulo 2^width
+            if (wrap) fset(k, f[1], (fget(k, f[1]) + 1) % 2);
+            })
             break;
-        }
-        case SQ_OP_BIT_GATHER: {
-            const uint64_t v = fget<K>(k, f[0]);
+        case SQ_OP_BIT_GATHER:
+            SQ_EACH({
+            const uint64_t v = fget(k, f[0]);
             const uint64_t set = in.imm[0], rest = wmask(f[0].width) & ~set;  // host: set below the width
             const unsigned ns = (unsigned)__popcll(set);
-            fset<K>(k, f[0], in.dag ? bits_deposit(v, set) | bits_deposit(shr(v, ns), rest)
+            fset(k, f[0], in.dag ? bits_deposit(v, set) | bits_deposit(shr(v, ns), rest)
                                     : bits_extract(v, set) | shl(bits_extract(v, rest), ns));
+            })
             break;
-        }
-        case SQ_OP_SUB_UINT_UINT: fset<K>(k, f[2], fget<K>(k, f[2]) ^ (fget<K>(k, f[0]) - fget<K>(k, f[1]))); break;
-        case SQ_OP_NEG_UINT: fset<K>(k, f[1], fget<K>(k, f[1]) ^ (0ull - fget<K>(k, f[0]))); break;
-        case SQ_OP_ABS_SINT: {
-            const int64_t v = sext(fget<K>(k, f[0]), f[0].width);
+        case SQ_OP_SUB_UINT_UINT: SQ_EACH(fset(k, f[2], fget(k, f[2]) ^ (fget(k, f[0]) - fget(k, f[1])));) break;
+        case SQ_OP_NEG_UINT: SQ_EACH(fset(k, f[1], fget(k, f[1]) ^ (0ull - fget(k, f[0])));) break;
+        case SQ_OP_ABS_SINT:
+            SQ_EACH({
+            const int64_t v = sext(fget(k, f[0]), f[0].width);
             const uint64_t mag = v < 0 ? (uint64_t)(-v) : (uint64_t)v;
-            fset<K>(k, f[1], fget<K>(k, f[1]) ^ mag);
+            fset(k, f[1], fget(k, f[1]) ^ mag);
+            })
             break;
-        }
-        case SQ_OP_MUL_UINT_UINT: fset<K>(k, f[2], fget<K>(k, f[2]) ^ (fget<K>(k, f[0]) * fget<K>(k, f[1]))); break;
-        case SQ_OP_DIV_UINT_UINT: {
-            const uint64_t x = fget<K>(k, f[0]), y = fget<K>(k, f[1]);
-            fset<K>(k, f[2], fget<K>(k, f[2]) ^ (y == 0 ? 0ull : x / y));
+        case SQ_OP_MUL_UINT_UINT: SQ_EACH(fset(k, f[2], fget(k, f[2]) ^ (fget(k, f[0]) * fget(k, f[1])));) break;
+        case SQ_OP_DIV_UINT_UINT:
+            SQ_EACH({
+            const uint64_t x = fget(k, f[0]), y = fget(k, f[1]);
+            fset(k, f[2], fget(k, f[2]) ^ (y == 0 ? 0ull : x / y));
+            })
             break;
-        }
-        case SQ_OP_SQRT_UINT: fset<K>(k, f[1], fget<K>(k, f[1]) ^ isqrt64(fget<K>(k, f[0]))); break;
-        case SQ_OP_SELECT_BOOL: {
-            const uint64_t sel = (fget<K>(k, f[0]) & 1ull) ? fget<K>(k, f[1]) : fget<K>(k, f[2]);
-            fset<K>(k, f[3], fget<K>(k, f[3]) ^ sel);
+        case SQ_OP_SQRT_UINT: SQ_EACH(fset(k, f[1], fget(k, f[1]) ^ isqrt64(fget(k, f[0])));) break;
+        case SQ_OP_SELECT_BOOL:
+            SQ_EACH({
+            const uint64_t sel = (fget(k, f[0]) & 1ull) ? fget(k, f[1]) : fget(k, f[2]);
+            fset(k, f[3], fget(k, f[3]) ^ sel);
+            })
             break;
-        }
-        case SQ_OP_AND_UINT_UINT: fset<K>(k, f[2], fget<K>(k, f[2]) ^ (fget<K>(k, f[0]) & fget<K>(k, f[1]))); break;
-        case SQ_OP_OR_UINT_UINT: fset<K>(k, f[2], fget<K>(k, f[2]) ^ (fget<K>(k, f[0]) | fget<K>(k, f[1]))); break;
-        case SQ_OP_XOR_UINT_UINT: fset<K>(k, f[2], fget<K>(k, f[2]) ^ (fget<K>(k, f[0]) ^ fget<K>(k, f[1]))); break;
-        case SQ_OP_LESS_SINT_SINT: {
-            const bool p = sext(fget<K>(k, f[0]), f[0].width) < sext(fget<K>(k, f[1]), f[1].width);
-            fset<K>(k, f[2], fget<K>(k, f[2]) ^ (p ? 1ull : 0ull));
+        case SQ_OP_AND_UINT_UINT: SQ_EACH(fset(k, f[2], fget(k, f[2]) ^ (fget(k, f[0]) & fget(k, f[1])));) break;
+        case SQ_OP_OR_UINT_UINT: SQ_EACH(fset(k, f[2], fget(k, f[2]) ^ (fget(k, f[0]) | fget(k, f[1])));) break;
+        case SQ_OP_XOR_UINT_UINT: SQ_EACH(fset(k, f[2], fget(k, f[2]) ^ (fget(k, f[0]) ^ fget(k, f[1])));) break;
+        case SQ_OP_LESS_SINT_SINT:
+            SQ_EACH({
+            const bool p = sext(fget(k, f[0]), f[0].width) < sext(fget(k, f[1]), f[1].width);
+            fset(k, f[2], fget(k, f[2]) ^ (p ? 1ull : 0ull));
+            })
             break;
-        }
-        case SQ_OP_CARRY_UINT_UINT: {
-            const uint64_t x = fget<K>(k, f[0]), y = fget<K>(k, f[1]);
+        case SQ_OP_CARRY_UINT_UINT:
+            SQ_EACH({
+            const uint64_t x = fget(k, f[0]), y = fget(k, f[1]);
             const unsigned w = f[2].width;
             const bool p = w >= 64 ? (x + y < x) : (x >= (1ull << w)) || (y >= (1ull << w) - x);
-            fset<K>(k, f[3], fget<K>(k, f[3]) ^ (p ? 1ull : 0ull));
+            fset(k, f[3], fget(k, f[3]) ^ (p ? 1ull : 0ull));
+            })
             break;
-        }
-        case SQ_OP_OVERFLOW_SINT_SINT: {
+        case SQ_OP_OVERFLOW_SINT_SINT:
+            SQ_EACH({
             const unsigned w = f[2].width;
             const uint64_t m = wmask(w);
-            const uint64_t A = (uint64_t)sext(fget<K>(k, f[0]), f[0].width) & m;
-            const uint64_t B = (uint64_t)sext(fget<K>(k, f[1]), f[1].width) & m;
+            const uint64_t A = (uint64_t)sext(fget(k, f[0]), f[0].width) & m;
+            const uint64_t B = (uint64_t)sext(fget(k, f[1]), f[1].width) & m;
             const uint64_t S = (A + B) & m;
             const uint64_t sa = (A >> (w - 1)) & 1, sb = (B >> (w - 1)) & 1, ss = (S >> (w - 1)) & 1;
             const bool p = (sa == sb) && (ss != sa);
-            fset<K>(k, f[3], fget<K>(k, f[3]) ^ (p ? 1ull : 0ull));
+            fset(k, f[3], fget(k, f[3]) ^ (p ? 1ull : 0ull));
+            })
             break;
-        }
-        case SQ_OP_MULOVERFLOW_UINT_UINT: {
-            const uint64_t x = fget<K>(k, f[0]), y = fget<K>(k, f[1]);
+        case SQ_OP_MULOVERFLOW_UINT_UINT:
+            SQ_EACH({
+            const uint64_t x = fget(k, f[0]), y = fget(k, f[1]);
             const uint64_t lo = x * y, hi = __umul64hi(x, y);
             const unsigned w = f[2].width;
             const bool p = hi != 0 || (w < 64 && lo >= (1ull << w));
-            fset<K>(k, f[3], fget<K>(k, f[3]) ^ (p ? 1ull : 0ull));
+            fset(k, f[3], fget(k, f[3]) ^ (p ? 1ull : 0ull));
+            })
             break;
-        }
-        case SQ_OP_ISZERO_UINT: fset<K>(k, f[1], fget<K>(k, f[1]) ^ (fget<K>(k, f[0]) == 0 ? 1ull : 0ull)); break;
-        case SQ_OP_NEGATIVE_SINT:
-            fset<K>(k, f[1], fget<K>(k, f[1]) ^ (sext(fget<K>(k, f[0]), f[0].width) < 0 ? 1ull : 0ull));
-            break;
-        case SQ_OP_ADD_ANYINT_INPLACE: {
-            const uint64_t raw = fget<K>(k, f[1]);
+        case SQ_OP_ISZERO_UINT: SQ_EACH(fset(k, f[1], fget(k, f[1]) ^ (fget(k, f[0]) == 0 ? 1ull : 0ull));) break;
+        case SQ_OP_NEGATIVE_SINT: SQ_EACH(fset(k, f[1], fget(k, f[1]) ^ (sext(fget(k, f[0]), f[0].width) < 0 ? 1ull : 0ull));) break;
+        case SQ_OP_ADD_ANYINT_INPLACE:
+            SQ_EACH({
+            const uint64_t raw = fget(k, f[1]);
             const uint64_t ext = f[1].type == SQ_SIGNED ? (uint64_t)sext(raw, f[1].width) : raw;
-            const uint64_t o = fget<K>(k, f[0]);
-            fset<K>(k, f[0], in.dag ? o - ext : o + ext);
+            const uint64_t o = fget(k, f[0]);
+            fset(k, f[0], in.dag ? o - ext : o + ext);
+            })
             break;
-        }
-        case SQ_OP_ASSIGN: fset<K>(k, f[1], fget<K>(k, f[1]) ^ fget<K>(k, f[0])); break;
-        case SQ_OP_COMPARE_UINT_UINT: {
-            const uint64_t l = fget<K>(k, f[0]), r = fget<K>(k, f[1]);
-            if (l == r) fset<K>(k, f[3], fget<K>(k, f[3]) ^ 1ull);
-            else fset<K>(k, f[2], fget<K>(k, f[2]) ^ (l < r ? 1ull : 0ull));
+        case SQ_OP_ASSIGN: SQ_EACH(fset(k, f[1], fget(k, f[1]) ^ fget(k, f[0]));) break;
+        case SQ_OP_COMPARE_UINT_UINT:
+            SQ_EACH({
+            const uint64_t l = fget(k, f[0]), r = fget(k, f[1]);
+            if (l == r) fset(k, f[3], fget(k, f[3]) ^ 1ull);
+            else fset(k, f[2], fget(k, f[2]) ^ (l < r ? 1ull : 0ull));
+            })
             break;
-        }
-        case SQ_OP_LESS_UINT_UINT:
-            fset<K>(k, f[2], fget<K>(k, f[2]) ^ (fget<K>(k, f[0]) < fget<K>(k, f[1]) ? 1ull : 0ull));
+        case SQ_OP_LESS_UINT_UINT: SQ_EACH(fset(k, f[2], fget(k, f[2]) ^ (fget(k, f[0]) < fget(k, f[1]) ? 1ull : 0ull));) break;
+        case SQ_OP_SWAP_GENERAL:
+            SQ_EACH({
+            const uint64_t x = fget(k, f[0]), y = fget(k, f[1]);
+            fset(k, f[0], y);
+            fset(k, f[1], x);
+            })
             break;
-        case SQ_OP_SWAP_GENERAL: {
-            const uint64_t x = fget<K>(k, f[0]), y = fget<K>(k, f[1]);
-            fset<K>(k, f[0], y);
-            fset<K>(k, f[1], x);
-            break;
-        }
-        case SQ_OP_GETMID_UINT_UINT:
-            fset<K>(k, f[2], fget<K>(k, f[2]) ^ ((fget<K>(k, f[0]) + fget<K>(k, f[1])) / 2));
-            break;
-        case SQ_OP_X_BOOL: fset<K>(k, f[0], fget<K>(k, f[0]) ^ (1ull << in.imm[0])); break;
-        case SQ_OP_INIT_UNSAFE: fset<K>(k, f[0], in.imm[0]); break;
-        case SQ_OP_QRAM_LOAD: {
-            const uint64_t addr = fget<K>(k, f[0]) & in.amask;
+        case SQ_OP_GETMID_UINT_UINT: SQ_EACH(fset(k, f[2], fget(k, f[2]) ^ ((fget(k, f[0]) + fget(k, f[1])) / 2));) break;
+        case SQ_OP_X_BOOL: SQ_EACH(fset(k, f[0], fget(k, f[0]) ^ (1ull << in.imm[0]));) break;
+        case SQ_OP_INIT_UNSAFE: SQ_EACH(fset(k, f[0], in.imm[0]);) break;
+        case SQ_OP_QRAM_LOAD:
+            SQ_EACH({
+            const uint64_t addr = fget(k, f[0]) & in.amask;
             uint64_t word;
             if (in.elem_bytes == 2) word = __ldg((const unsigned short*)in.table + addr);
             else if (in.elem_bytes == 4) word = __ldg((const unsigned int*)in.table + addr);
             else word = __ldg((const unsigned long long*)in.table + addr);
-            fset<K>(k, f[1], fget<K>(k, f[1]) ^ word);
+            fset(k, f[1], fget(k, f[1]) ^ word);
+            })
             break;
-        }
-        case SQ_OP_ADDR_XOR: {
-            uint64_t v = fget<K>(k, f[0]) + in.imm[0] * fget<K>(k, f[1]);
-            if (in.imm[1]) v += fget<K>(k, f[2]);
-            fset<K>(k, f[3], fget<K>(k, f[3]) ^ v);
+        case SQ_OP_ADDR_XOR:
+            SQ_EACH({
+            uint64_t v = fget(k, f[0]) + in.imm[0] * fget(k, f[1]);
+            if (in.imm[1]) v += fget(k, f[2]);
+            fset(k, f[3], fget(k, f[3]) ^ v);
+            })
             break;
-        }
-        case SQ_OP_QBS_XOR: {
+        case SQ_OP_QBS_XOR:
+            SQ_EACH({
             const uint64_t amask = wmask(in.addr_bits);
-            const uint64_t target = fget<K>(k, f[1]);
-            uint64_t l = fget<K>(k, f[0]), r = l + in.imm[0], found = 0;
+            const uint64_t target = fget(k, f[1]);
+            uint64_t l = fget(k, f[0]), r = l + in.imm[0], found = 0;
             for (uint64_t i = 0; i < in.imm[1]; ++i) {
                 const uint64_t mid = (l + r) / 2;
                 uint64_t word;
@@ -326,35 +364,38 @@ __device__ __forceinline__ void exec(const DInstr& in, uint64_t (&k)[K], double2
                 if (word < target) l = mid;
                 else r = mid;
             }
-            fset<K>(k, f[2], fget<K>(k, f[2]) ^ found);
+            fset(k, f[2], fget(k, f[2]) ^ found);
+            })
             break;
-        }
-        case SQ_OP_TRIDIAG_ELEMENT: {
-            const uint64_t idx = fget<K>(k, f[0]) + 4 * fget<K>(k, f[1]) + fget<K>(k, f[2]);
-            fset<K>(k, f[3], fget<K>(k, f[3]) ^ tri_mem(idx, in.imm[0], in.imm[1]));
+        case SQ_OP_TRIDIAG_ELEMENT:
+            SQ_EACH({
+            const uint64_t idx = fget(k, f[0]) + 4 * fget(k, f[1]) + fget(k, f[2]);
+            fset(k, f[3], fget(k, f[3]) ^ tri_mem(idx, in.imm[0], in.imm[1]));
+            })
             break;
-        }
-        case SQ_OP_TRIDIAG_SLOT_COLUMN: {
+        case SQ_OP_TRIDIAG_SLOT_COLUMN:
+            SQ_EACH({
             const uint64_t n = in.imm[0], kmask = wmask((unsigned)in.imm[2]);
-            const uint64_t j = fget<K>(k, f[1]), kv = fget<K>(k, f[2]), sr = fget<K>(k, f[3]) & kmask;
-            const uint64_t base = tri_window_base(j, n), row = fget<K>(k, f[0]) + 4 * j;
+            const uint64_t j = fget(k, f[1]), kv = fget(k, f[2]), sr = fget(k, f[3]) & kmask;
+            const uint64_t base = tri_window_base(j, n), row = fget(k, f[0]) + 4 * j;
             if (!in.dag) {  // column -> slot; out-of-window branches tagged into the tag register
                 const bool hit = kv >= base && kv < base + 4;
                 const uint64_t sr1 = sr ^ (hit ? row + (kv - base) : 0ull);
                 const uint64_t k1 = kv ^ tri_mem(sr1, n, in.imm[1]);
-                fset<K>(k, f[2], (sr1 - row) & kmask);
-                fset<K>(k, f[3], k1 & kmask);
+                fset(k, f[2], (sr1 - row) & kmask);
+                fset(k, f[3], k1 & kmask);
             } else {  // slot -> column
                 const uint64_t k1 = (kv + row) & kmask;
                 const uint64_t k2 = sr ^ tri_mem(k1, n, in.imm[1]);
                 const bool hit = k2 >= base && k2 < base + 4;
-                fset<K>(k, f[2], k2);
-                fset<K>(k, f[3], k1 ^ (hit ? row + (k2 - base) : 0ull));
+                fset(k, f[2], k2);
+                fset(k, f[3], k1 ^ (hit ? row + (k2 - base) : 0ull));
             }
+            })
             break;
-        }
-        case SQ_OP_LOOKUP_XOR: {
-            const uint64_t v = fget<K>(k, f[0]);
+        case SQ_OP_LOOKUP_XOR:
+            SQ_EACH({
+            const uint64_t v = fget(k, f[0]);
             const uint64_t* t = static_cast<const uint64_t*>(in.table);
             const uint64_t nd = in.imm[0], ns = in.imm[1];
             uint64_t w = 0;
@@ -370,14 +411,13 @@ __device__ __forceinline__ void exec(const DInstr& in, uint64_t (&k)[K], double2
                 if (lo < ns && __ldg(t + nd + lo) == v) w = __ldg(t + nd + ns + lo);
                 else atomicOr(err, 8u);
             }
-            fset<K>(k, f[1], fget<K>(k, f[1]) ^ w);
+            fset(k, f[1], fget(k, f[1]) ^ w);
+            })
             break;
-        }
-        case SQ_OP_PARITY_PHASE:
-            if (fget<K>(k, f[0]) & 1ull) a = make_double2(-a.x, -a.y);
-            break;
-        case SQ_OP_ANGLE_XOR: {
-            const uint64_t l = fget<K>(k, f[0]), r = fget<K>(k, f[1]);
+        case SQ_OP_PARITY_PHASE: SQ_EACH(if (fget(k, f[0]) & 1ull) a = make_double2(-a.x, -a.y);) break;
+        case SQ_OP_ANGLE_XOR:
+            SQ_EACH({
+            const uint64_t l = fget(k, f[0]), r = fget(k, f[1]);
             const uint64_t* t = static_cast<const uint64_t*>(in.table);
             const uint64_t mask = in.imm[0];
             const unsigned probes = (unsigned)in.imm[1];
@@ -395,42 +435,39 @@ __device__ __forceinline__ void exec(const DInstr& in, uint64_t (&k)[K], double2
                 if (x == ~0ull && y == ~0ull) break;
             }
             if (!found) atomicOr(err, 64u);
-            fset<K>(k, f[2], fget<K>(k, f[2]) ^ w);
+            fset(k, f[2], fget(k, f[2]) ^ w);
+            })
             break;
-        }
-        case SQ_OP_PHASE_BOOL:
-            if ((fget<K>(k, f[0]) >> in.imm[0]) & 1ull) a = cmul(a, in.c[0]);
-            break;
-        case SQ_OP_GLOBAL_PHASE: a = cmul(a, in.c[0]); break;
-        case SQ_OP_Y_BOOL: {
-            const uint64_t v = fget<K>(k, f[0]) ^ (1ull << in.imm[0]);
-            fset<K>(k, f[0], v);
+        case SQ_OP_PHASE_BOOL: SQ_EACH(if ((fget(k, f[0]) >> in.imm[0]) & 1ull) a = cmul(a, in.c[0]);) break;
+        case SQ_OP_GLOBAL_PHASE: SQ_EACH(a = cmul(a, in.c[0]);) break;
+        case SQ_OP_Y_BOOL:
+            SQ_EACH({
+            const uint64_t v = fget(k, f[0]) ^ (1ull << in.imm[0]);
+            fset(k, f[0], v);
             a = cmul(a, ((v >> in.imm[0]) & 1ull) ? make_double2(0.0, 1.0) : make_double2(0.0, -1.0));
+            })
             break;
-        }
         case SQ_OP_REFLECTION_BOOL:
-        case SQ_OP_ZERO_COND_PHASE_FLIP: {
-            bool iszero = true;
-#pragma unroll
-            for (int w = 0; w < K; ++w) iszero = iszero && ((k[w] & in.zmask[w]) == 0);
+        case SQ_OP_ZERO_COND_PHASE_FLIP:
+            SQ_EACH({
+            const bool iszero = all_zero(k, in.zmask);
             bool flip = in.op == SQ_OP_ZERO_COND_PHASE_FLIP ? iszero : !((in.imm[1] != 0) ^ iszero);
             if (flip) a = make_double2(a.x * -1.0, a.y * -1.0);
+            })
             break;
-        }
-        case SQ_OP_ROT_DIAGONAL:
-            a = cmul(a, ((fget<K>(k, f[0]) >> in.imm[0]) & 1ull) ? in.c[1] : in.c[0]);
-            break;
-        case SQ_OP_ROT_OFF_DIAGONAL: {
-            const uint64_t v = fget<K>(k, f[0]);
+        case SQ_OP_ROT_DIAGONAL: SQ_EACH(a = cmul(a, ((fget(k, f[0]) >> in.imm[0]) & 1ull) ? in.c[1] : in.c[0]);) break;
+        case SQ_OP_ROT_OFF_DIAGONAL:
+            SQ_EACH({
+            const uint64_t v = fget(k, f[0]);
             a = cmul(a, ((v >> in.imm[0]) & 1ull) ? in.c[1] : in.c[0]);
-            fset<K>(k, f[0], v ^ (1ull << in.imm[0]));
+            fset(k, f[0], v ^ (1ull << in.imm[0]));
+            })
             break;
-        }
-        case SQ_OP_PAULI_NOISE: {
-            const uint64_t t = fget<K>(k, f[0]);
-            if (t >= in.imm[0]) break;
+        case SQ_OP_PAULI_NOISE:
+            SQ_EACH({
+            const uint64_t t = fget(k, f[0]);
+            if (t >= in.imm[0]) continue;
             uint64_t m[6];
-#pragma unroll
             for (int r = 0; r < 6; ++r) {
                 const uint64_t idx = t * 6 + r;
                 if (in.elem_bytes == 2) m[r] = __ldg((const unsigned short*)in.table + idx);
@@ -438,54 +475,213 @@ __device__ __forceinline__ void exec(const DInstr& in, uint64_t (&k)[K], double2
                 else m[r] = __ldg((const unsigned long long*)in.table + idx);
             }
             int parity = 0;
-#pragma unroll
             for (int r = 0; r < 3; ++r) {
-                const uint64_t v = fget<K>(k, f[r + 1]) ^ m[r];
-                fset<K>(k, f[r + 1], v);
+                const uint64_t v = fget(k, f[r + 1]) ^ m[r];
+                fset(k, f[r + 1], v);
                 parity += __popcll(v & m[r + 3]);
             }
             if (parity & 1) a = make_double2(a.x * -1.0, a.y * -1.0);
+            })
             break;
-        }
         default: break;
     }
 }
 
-template <int K, int MAXI>
-__global__ void __launch_bounds__(256) program_kernel(const __grid_constant__ ProgramArgs<MAXI> p, KeyPtrs keys,
+// The same for the common operators when every field is at most 32 bits wide:
+// results are kept modulo 2^32 or less, so 32-bit arithmetic gives the same
+// bits, and a field costs one funnel shift and one AND. The first 8 bytes of a
+// field (word, shift, mask) are one constant load. A 9-operator chain over
+// 32-bit registers, 2^23 entries of two key words: 215 us in 64-bit arithmetic,
+// 165 here; both are bound by integer issue (the ALU pipe 69 to 75 % busy).
+// Keeping the fields in shared-memory slots while a program runs was measured
+// too (205 us).
+struct NField {
+    unsigned word, shift;
+    uint32_t mask;
+};
+__device__ __forceinline__ NField nfield(const DField& f) {
+    const uint2 r = *reinterpret_cast<const uint2*>(&f);
+    return NField{r.x & 0xffu, (r.x >> 8) & 0xffu, r.y};
+}
+template <int K>
+__device__ __forceinline__ uint32_t nget(const WordRegs<K>& r, const NField& f) {
+    return (uint32_t)(kword<K>(r.k, f.word) >> f.shift) & f.mask;
+}
+template <int K>
+__device__ __forceinline__ void nset(WordRegs<K>& r, const NField& f, uint32_t v) {
+    const uint64_t w = kword<K>(r.k, f.word);
+    kword_set<K>(r.k, f.word, (w & ~((uint64_t)f.mask << f.shift)) | ((uint64_t)(v & f.mask) << f.shift));
+}
+// f ^= v
+template <int K>
+__device__ __forceinline__ void nxor(WordRegs<K>& r, const NField& f, uint32_t v) {
+    kword_set<K>(r.k, f.word, kword<K>(r.k, f.word) ^ ((uint64_t)(v & f.mask) << f.shift));
+}
+__device__ __forceinline__ uint32_t shl32(uint32_t v, unsigned s) { return s >= 32 ? 0u : v << s; }
+__device__ __forceinline__ uint32_t shr32(uint32_t v, unsigned s) { return s >= 32 ? 0u : v >> s; }
+
+template <typename R, int Q>
+__device__ __forceinline__ void exec_narrow(const DInstr& in, R (&kk)[Q], double2 (&aa)[Q], const bool (&ok)[Q]) {
+    const NField f[4] = {nfield(in.f[0]), nfield(in.f[1]), nfield(in.f[2]), nfield(in.f[3])};
+    const uint32_t imm = (uint32_t)in.imm[0];
+    switch (in.op) {
+        case SQ_OP_FLIP_BOOLS: SQ_EACH(nxor(k, f[0], 0xffffffffu);) break;
+        case SQ_OP_SHIFT_LEFT:
+        case SQ_OP_SHIFT_RIGHT: {
+            const unsigned size = in.f[0].width;
+            const bool left = (in.op == SQ_OP_SHIFT_LEFT) != (in.dag != 0);
+            const unsigned d = left ? imm : size - imm;  // a right rotation by d is a left one by size - d
+            SQ_EACH(const uint32_t v = nget(k, f[0]); nset(k, f[0], shl32(v, d) | shr32(v, size - d));)
+            break;
+        }
+        case SQ_OP_MULT_UINT_CONST: SQ_EACH(nxor(k, f[2], nget(k, f[0]) * imm);) break;
+        case SQ_OP_ADD_MULT_UINT_CONST:
+            SQ_EACH(nset(k, f[2], nget(k, f[2]) + nget(k, f[0]) * (in.dag ? 0u - imm : imm));)
+            break;
+        case SQ_OP_ADD_UINT_UINT: SQ_EACH(nxor(k, f[2], nget(k, f[0]) + nget(k, f[1]));) break;
+        case SQ_OP_SUB_UINT_UINT: SQ_EACH(nxor(k, f[2], nget(k, f[0]) - nget(k, f[1]));) break;
+        case SQ_OP_MUL_UINT_UINT: SQ_EACH(nxor(k, f[2], nget(k, f[0]) * nget(k, f[1]));) break;
+        case SQ_OP_AND_UINT_UINT: SQ_EACH(nxor(k, f[2], nget(k, f[0]) & nget(k, f[1]));) break;
+        case SQ_OP_OR_UINT_UINT: SQ_EACH(nxor(k, f[2], nget(k, f[0]) | nget(k, f[1]));) break;
+        case SQ_OP_XOR_UINT_UINT: SQ_EACH(nxor(k, f[2], nget(k, f[0]) ^ nget(k, f[1]));) break;
+        case SQ_OP_LESS_UINT_UINT: SQ_EACH(nxor(k, f[2], nget(k, f[0]) < nget(k, f[1]) ? 1u : 0u);) break;
+        case SQ_OP_ADD_UINT_UINT_INPLACE:
+            SQ_EACH(const uint32_t l = nget(k, f[0]); nset(k, f[1], nget(k, f[1]) + (in.dag ? 0u - l : l));)
+            break;
+        case SQ_OP_ADD_UINT_CONST: SQ_EACH(nxor(k, f[2], nget(k, f[0]) + imm);) break;
+        case SQ_OP_ADD_CONST_INPLACE: SQ_EACH(nset(k, f[0], nget(k, f[0]) + (in.dag ? 0u - imm : imm));) break;
+        case SQ_OP_NEG_UINT: SQ_EACH(nxor(k, f[1], 0u - nget(k, f[0]));) break;
+        case SQ_OP_ISZERO_UINT: SQ_EACH(nxor(k, f[1], nget(k, f[0]) == 0u ? 1u : 0u);) break;
+        case SQ_OP_ASSIGN: SQ_EACH(nxor(k, f[1], nget(k, f[0]));) break;
+        case SQ_OP_SWAP_GENERAL:
+            SQ_EACH(const uint32_t x = nget(k, f[0]); const uint32_t y = nget(k, f[1]); nset(k, f[0], y);
+                    nset(k, f[1], x);)
+            break;
+        case SQ_OP_X_BOOL: SQ_EACH(nxor(k, f[0], 1u << imm);) break;
+        case SQ_OP_INIT_UNSAFE: SQ_EACH(nset(k, f[0], imm);) break;
+        case SQ_OP_QRAM_LOAD: {
+            uint32_t w[Q];  // the loads of all entries before the first use
+            SQ_EACH({
+                const uint32_t addr = nget(k, f[0]) & (uint32_t)in.amask;
+                if (in.elem_bytes == 2) w[q] = __ldg((const unsigned short*)in.table + addr);
+                else if (in.elem_bytes == 4) w[q] = __ldg((const unsigned int*)in.table + addr);
+                else w[q] = (uint32_t)__ldg((const unsigned long long*)in.table + addr);
+            })
+            SQ_EACH(nxor(k, f[1], w[q]);)
+            break;
+        }
+        case SQ_OP_ADDR_XOR:
+            SQ_EACH({
+                uint32_t v = nget(k, f[0]) + imm * nget(k, f[1]);
+                if (in.imm[1]) v += nget(k, f[2]);
+                nxor(k, f[3], v);
+            })
+            break;
+        default: break;
+    }
+}
+#undef SQ_EACH
+
+// Whether an instruction may take exec_narrow (its cases above).
+static bool narrow_ok(const DInstr& d) {
+    for (const DField& f : d.f)
+        if (f.width > 32) return false;
+    switch (d.op) {
+        case SQ_OP_FLIP_BOOLS: case SQ_OP_SHIFT_LEFT: case SQ_OP_SHIFT_RIGHT: case SQ_OP_MULT_UINT_CONST:
+        case SQ_OP_ADD_MULT_UINT_CONST: case SQ_OP_ADD_UINT_UINT: case SQ_OP_SUB_UINT_UINT: case SQ_OP_MUL_UINT_UINT:
+        case SQ_OP_AND_UINT_UINT: case SQ_OP_OR_UINT_UINT: case SQ_OP_XOR_UINT_UINT: case SQ_OP_LESS_UINT_UINT:
+        case SQ_OP_ADD_UINT_UINT_INPLACE: case SQ_OP_ADD_UINT_CONST: case SQ_OP_ADD_CONST_INPLACE: case SQ_OP_NEG_UINT:
+        case SQ_OP_ISZERO_UINT: case SQ_OP_ASSIGN: case SQ_OP_SWAP_GENERAL: case SQ_OP_X_BOOL: case SQ_OP_INIT_UNSAFE:
+        case SQ_OP_QRAM_LOAD: case SQ_OP_ADDR_XOR: return true;
+        default: return false;
+    }
+}
+
+// The key words a program uses, in the order of their local numbers (the
+// words of fields and conditions are renumbered on the host): a program that
+// touches 2 of 6 key words holds and selects among 2.
+struct LocalKeys {
+    uint64_t* w[SQ_KMAX];
+};
+
+// Q consecutive entries per thread, moved by 16-byte accesses when Q is even:
+// the interpreter's share (decoding, field and condition parameters) is paid
+// once for them and their loads are in flight together.
+template <int K, int Q, int MAXI>
+__global__ void __launch_bounds__(256) program_kernel(const __grid_constant__ ProgramArgs<MAXI> p, LocalKeys keys,
                                                       double2* __restrict__ amp, uint64_t n) {
     // warp-uniform trips (the entry index is per lane, the loop is not), so
     // that the instruction index is uniform and the instruction's fields are
     // uniform loads
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x; b < n; b += stride) {
-        const uint64_t i = b + threadIdx.x;
-        const bool valid = i < n;
-        uint64_t k[K];
+    const uint64_t stride = (uint64_t)gridDim.x * (256u * Q);
+    for (uint64_t b = (uint64_t)blockIdx.x * (256u * Q); b < n; b += stride) {
+        const uint64_t i = b + (uint64_t)threadIdx.x * Q;
+        const bool whole = i + Q <= n;
+        WordRegs<K> k[Q];
+        double2 a[Q];
 #pragma unroll
-        for (int w = 0; w < K; ++w) k[w] = (valid && ((p.read_words >> w) & 1u)) ? keys.w[w][i] : 0ull;
-        double2 a = make_double2(0.0, 0.0);
-        if (valid && (p.amp_mode & 1u)) a = amp[i];
+        for (int q = 0; q < Q; ++q) a[q] = make_double2(0.0, 0.0);
+        if (Q > 1 && whole) {
+#pragma unroll
+            for (int w = 0; w < K; ++w)
+#pragma unroll
+                for (int q = 0; q + 1 < Q; q += 2) {
+                    if (!((p.read_words >> w) & 1u)) {
+                        k[q].k[w] = k[q + 1].k[w] = 0ull;
+                        continue;
+                    }
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(keys.w[w] + i + q);
+                    k[q].k[w] = v.x;
+                    k[q + 1].k[w] = v.y;
+                }
+            if (p.amp_mode & 1u)
+#pragma unroll
+                for (int q = 0; q < Q; ++q) a[q] = amp[i + q];
+        } else {
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+#pragma unroll
+                for (int w = 0; w < K; ++w) k[q].k[w] = (i + q < n && ((p.read_words >> w) & 1u)) ? keys.w[w][i + q] : 0ull;
+                if (i + q < n && (p.amp_mode & 1u)) a[q] = amp[i + q];
+            }
+        }
         for (uint32_t j = 0; j < p.n; ++j) {
             const DInstr& in = p.ins[j];
-            if (valid && cond_ok<K>(k, in.cond)) exec<K>(in, k, a, p.err);
-        }
-        if (!valid) continue;
+            bool ok[Q];
 #pragma unroll
-        for (int w = 0; w < K; ++w)
-            if ((p.write_words >> w) & 1u) keys.w[w][i] = k[w];
-        if (p.amp_mode & 2u) amp[i] = a;
+            for (int q = 0; q < Q; ++q) ok[q] = i + q < n && holds(k[q], in.cond);
+            if (in.narrow) exec_narrow<WordRegs<K>, Q>(in, k, a, ok);
+            else exec<WordRegs<K>, Q>(in, k, a, ok, p.err);
+        }
+        if (Q > 1 && whole) {
+#pragma unroll
+            for (int w = 0; w < K; ++w) {
+                if (!((p.write_words >> w) & 1u)) continue;
+#pragma unroll
+                for (int q = 0; q + 1 < Q; q += 2)
+                    *reinterpret_cast<ulonglong2*>(keys.w[w] + i + q) = make_ulonglong2(k[q].k[w], k[q + 1].k[w]);
+            }
+            if (p.amp_mode & 2u)
+#pragma unroll
+                for (int q = 0; q < Q; ++q) amp[i + q] = a[q];
+        } else {
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                if (i + q >= n) continue;
+#pragma unroll
+                for (int w = 0; w < K; ++w)
+                    if ((p.write_words >> w) & 1u) keys.w[w][i + q] = k[q].k[w];
+                if (p.amp_mode & 2u) amp[i + q] = a[q];
+            }
+        }
     }
 }
 
-template <int K, int MAXI>
-static void launch_program(const ProgramArgs<MAXI>& args, State& s, double table_bytes) {
-    KeyPtrs kp;
-    for (int w = 0; w < SQ_KMAX; ++w) kp.w[w] = s.live.keys[w];
-    const int block = 256;
-    unsigned grid = grid_for(s.n, block, 8);
+template <int K, int Q, int MAXI>
+static void launch_program(const ProgramArgs<MAXI>& args, const LocalKeys& keys, State& s, double table_bytes) {
+    unsigned grid = grid_for((s.n + Q - 1) / Q, 256, 8);
     prof_begin("elementwise_program");
-    program_kernel<K, MAXI><<<grid, block, 0, stream()>>>(args, kp, s.live.amp, s.n);
+    program_kernel<K, Q, MAXI><<<grid, 256, 0, stream()>>>(args, keys, s.live.amp, s.n);
     // compulsory traffic: words read + words written + amplitude in/out + table words touched
     const double per = 8.0 * __builtin_popcount(args.read_words) + 8.0 * __builtin_popcount(args.write_words) +
                        16.0 * (args.amp_mode & 1u) + 16.0 * ((args.amp_mode >> 1) & 1u);
@@ -493,23 +689,58 @@ static void launch_program(const ProgramArgs<MAXI>& args, State& s, double table
     SQ_CUDA(cudaGetLastError());
 }
 
+template <int K, int MAXI>
+static void dispatch_q(const ProgramArgs<MAXI>& args, const LocalKeys& keys, State& s, double tb) {
+    // two entries per thread once that still gives every SM its warps (four
+    // were slower at two key words, 185 against 165 us for the chain above)
+    constexpr int Q = 2;
+    if (s.n >= (uint64_t)num_sms() * 2048 * Q) launch_program<K, Q, MAXI>(args, keys, s, tb);
+    else launch_program<K, 1, MAXI>(args, keys, s, tb);
+}
+
+// Renumbers the key words of a translated program to the words that it uses.
 template <int MAXI>
-static void dispatch_k(const ProgramArgs<MAXI>& args, State& s, uint32_t k) {
+static uint32_t localise(ProgramArgs<MAXI>& args, const State& s, LocalKeys& keys) {
+    uint8_t local[SQ_KMAX] = {0};
+    uint32_t nl = 0, writes = 0;
+    memset(&keys, 0, sizeof(keys));
+    for (uint32_t w = 0; w < SQ_KMAX; ++w) {
+        if (!((args.read_words >> w) & 1u)) continue;
+        local[w] = (uint8_t)nl;
+        if ((args.write_words >> w) & 1u) writes |= 1u << nl;
+        keys.w[nl++] = s.live.keys[w];
+    }
+    for (uint32_t i = 0; i < args.n; ++i) {
+        DInstr& d = args.ins[i];
+        for (DField& f : d.f) f.word = local[f.word];
+        for (uint32_t j = 0; j < d.cond.n; ++j) d.cond.c[j].word = local[d.cond.c[j].word];
+        uint64_t z[SQ_KMAX] = {0};
+        for (uint32_t w = 0; w < SQ_KMAX; ++w)
+            if (d.zmask[w]) z[local[w]] = d.zmask[w];
+        memcpy(d.zmask, z, sizeof(z));
+    }
+    args.read_words = (1u << nl) - 1u;
+    args.write_words = writes;
+    return nl;
+}
+
+template <int MAXI>
+static void dispatch_k(ProgramArgs<MAXI>& args, State& s) {
     double tb = 0.0;
     for (uint32_t i = 0; i < args.n; ++i)
         if (args.ins[i].op == SQ_OP_QRAM_LOAD) {
             const double words = (double)(1ull << args.ins[i].addr_bits);
             tb += std::min((double)s.n, words) * args.ins[i].elem_bytes;
         }
-    switch (k) {
-        case 1: launch_program<1, MAXI>(args, s, tb); break;
-        case 2: launch_program<2, MAXI>(args, s, tb); break;
-        case 3: launch_program<3, MAXI>(args, s, tb); break;
-        case 4: launch_program<4, MAXI>(args, s, tb); break;
-        case 5: launch_program<5, MAXI>(args, s, tb); break;
-        case 6: launch_program<6, MAXI>(args, s, tb); break;
-        case 7: launch_program<7, MAXI>(args, s, tb); break;
-        default: launch_program<8, MAXI>(args, s, tb); break;
+    LocalKeys keys;
+    const uint32_t nl = localise(args, s, keys);
+    switch (nl) {
+        case 0:  // amplitudes only
+        case 1: dispatch_q<1, MAXI>(args, keys, s, tb); break;
+        case 2: dispatch_q<2, MAXI>(args, keys, s, tb); break;
+        case 3: dispatch_q<3, MAXI>(args, keys, s, tb); break;
+        case 4: dispatch_q<4, MAXI>(args, keys, s, tb); break;
+        default: launch_program<8, 1, MAXI>(args, keys, s, tb); break;  // 5 to 8 words
     }
 }
 
@@ -744,13 +975,13 @@ static void translate(const sq_instr& in, DInstr& d, uint32_t& rw, uint32_t& ww,
         default: fail(SQ_ERR_INVALID, "unknown opcode " + std::to_string(in.op));
     }
     d.amask = wmask(d.addr_bits);
+    d.narrow = narrow_ok(d) ? 1 : 0;
 }
 
 void run_program(State& s, const sq_instr* prog, uint32_t n) {
     if (n == 0) return;
     if (n > SQ_MAX_PROGRAM) fail(SQ_ERR_CAPACITY, "program longer than SQ_MAX_PROGRAM");
     uint32_t rw = 0, ww = 0, am = 0;
-    uint32_t k = regtable().k;
     sync_words(s);
     if (s.n == 0) {
         // still validate arguments like the reference constructors would
@@ -768,7 +999,7 @@ void run_program(State& s, const sq_instr* prog, uint32_t n) {
         a.write_words = ww;
         a.amp_mode = am;
         if (ww) drop_groups(s);  // key values change: cached group ranges no longer hold
-        dispatch_k<4>(a, s, k);
+        dispatch_k<4>(a, s);
     } else {
         ProgramArgs<SQ_MAX_PROGRAM>* a = new ProgramArgs<SQ_MAX_PROGRAM>;
         memset(a, 0, sizeof(*a));
@@ -784,7 +1015,7 @@ void run_program(State& s, const sq_instr* prog, uint32_t n) {
         a->write_words = ww;
         a->amp_mode = am;
         if (ww) drop_groups(s);
-        dispatch_k<SQ_MAX_PROGRAM>(*a, s, k);
+        dispatch_k<SQ_MAX_PROGRAM>(*a, s);
         delete a;
     }
 }

@@ -3613,7 +3613,7 @@ static void split_features(State& s, const GroupSpec& gs, uint64_t N, const uint
     f[10] = (float)(std::log2((double)N) / 32.0);
     f[11] = cached ? 1.f : 0.f;
     f[12] = cached ? (float)(std::log2((double)cached_groups + 1.0) / 32.0) : 0.f;
-    f[13] = (float)gs.cond.n / 8.f;
+    f[13] = (float)gs.cond.asked / 8.f;
     f[15] = 1.f;
     cudaStream_t st = stream();
     unsigned* regs = (unsigned*)ws().get(WS_SKETCH, 32 * 4);
@@ -3795,7 +3795,7 @@ static void run_group(State& s, const GroupSpec& gs) {
     uint64_t tune_key = 0;
     const bool tuned = strat == 3 && gs.mode != GM_MERGE && !gs.varw.width && N >= 4096;
     if (tuned) {
-        tune_key = (uint64_t)gs.mode | ((uint64_t)gs.cond.n << 8) | ((uint64_t)K << 16) |
+        tune_key = (uint64_t)gs.mode | ((uint64_t)gs.cond.asked << 8) | ((uint64_t)K << 16) |
                    ((uint64_t)(63 - __builtin_clzll(N)) << 24);
         strat = autotune_pick(tune_key);
     } else if (strat == 3) {

@@ -119,18 +119,35 @@ DCondSet resolve_cond(const sq_cond* c) {
     memset(&d, 0, sizeof(d));
     if (!c) return d;
     if (c->count > SQ_MAX_CONDITIONS) fail(SQ_ERR_INVALID, "too many conditions");
-    d.n = c->count;
+    d.asked = c->count;
     for (uint32_t i = 0; i < c->count; ++i) {
         const sq_condition& q = c->c[i];
         if (q.kind > SQ_COND_VALUE) fail(SQ_ERR_INVALID, "bad condition kind");
         Field f = regtable().field(q.reg);
-        d.c[i].kind = (uint8_t)q.kind;
-        d.c[i].word = f.word;
-        d.c[i].shift = f.shift;
-        d.c[i].width = f.width;
-        d.c[i].mask = wmask(f.width);
-        d.c[i].param = q.param;
         if (q.kind == SQ_COND_BIT && q.param >= 64) fail(SQ_ERR_INVALID, "condition bit >= 64");
+        const uint64_t m = wmask(f.width);
+        DCond t{m << f.shift, 0, f.word, 0};
+        if (q.kind == SQ_COND_NONZERO) {
+            t.ne = 1;
+        } else {
+            const uint64_t want = q.kind == SQ_COND_ALL_ONES ? m : q.kind == SQ_COND_BIT ? 1ull << q.param : q.param;
+            if (q.kind == SQ_COND_BIT) t.mask = (want & m) << f.shift;
+            t.val = (want & m) << f.shift;
+            if (want & ~m) {  // a value or bit that the register cannot hold: never true
+                t.mask = 0;
+                t.val = 1;
+            }
+        }
+        bool merged = false;
+        for (uint32_t j = 0; j < d.n && !t.ne && !merged; ++j) {
+            DCond& o = d.c[j];
+            if (o.ne || o.word != t.word || ((o.val ^ t.val) & o.mask & t.mask)) continue;
+            if ((o.val & ~o.mask) || (t.val & ~t.mask)) continue;  // never true: kept as it is
+            o.mask |= t.mask;
+            o.val |= t.val;
+            merged = true;
+        }
+        if (!merged) d.c[d.n++] = t;
     }
     return d;
 }

@@ -101,18 +101,19 @@ struct RegTable {
 RegTable& regtable();
 
 // ------------------------------------------------------------------ conditions
+// A condition is a masked compare of one key word, (key & mask) == val, or !=
+// when ne is set. Conditions on the same word that ask for given bits are
+// merged into one on the host, so that an operator controlled by several
+// registers usually tests one word once.
 struct DCond {
-    uint8_t kind;
-    uint8_t word;
-    uint8_t shift;
-    uint8_t width;
-    uint32_t pad;
-    uint64_t param;
-    uint64_t mask;  // wmask(width), computed on the host
+    uint64_t mask;
+    uint64_t val;
+    uint32_t word;
+    uint32_t ne;
 };
 struct DCondSet {
     uint32_t n;
-    uint32_t pad;
+    uint32_t asked;  // conditions as the caller gave them
     DCond c[SQ_MAX_CONDITIONS];
 };
 
@@ -146,13 +147,7 @@ __device__ __forceinline__ bool cond_ok(const uint64_t (&k)[K], const DCondSet& 
     bool ok = true;
     for (uint32_t i = 0; i < cs.n; ++i) {
         const DCond& c = cs.c[i];
-        const uint64_t v = (kword<K>(k, c.word) >> c.shift) & c.mask;
-        switch (c.kind) {
-            case SQ_COND_NONZERO: ok = ok && (v != 0); break;
-            case SQ_COND_ALL_ONES: ok = ok && (v == c.mask); break;
-            case SQ_COND_BIT: ok = ok && (c.param < 64) && ((v >> c.param) & 1ull); break;
-            default: ok = ok && (v == c.param); break;
-        }
+        ok = ok && (((kword<K>(k, c.word) & c.mask) == c.val) != (c.ne != 0));
     }
     return ok;
 }
