@@ -255,6 +255,11 @@ int sq_system_remove_register(uint32_t id);
 int sq_system_register_info(uint32_t id, uint32_t* type, uint32_t* width, uint32_t* active,
                             uint32_t* word, uint32_t* shift);
 int sq_system_register_count(uint32_t* n);
+/* The whole table at once: per register id five words (type, width, active,
+ * word, shift) into rows[5 * max_regs], the number of ids in *n, and (unless
+ * null) the address of a counter that changes whenever the table may have
+ * changed, for callers that keep a copy. */
+int sq_system_snapshot(uint32_t* rows, uint32_t max_regs, uint32_t* n, const uint64_t** changes);
 int sq_system_key_words(uint32_t* k);
 int sq_system_set_register_type(uint32_t id, uint32_t type);
 

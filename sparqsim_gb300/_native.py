@@ -92,6 +92,7 @@ _SIGS = [
     ("sq_system_remove_register", c_int, [c_uint32]),
     ("sq_system_register_info", c_int, [c_uint32] + [POINTER(c_uint32)] * 5),
     ("sq_system_register_count", c_int, [POINTER(c_uint32)]),
+    ("sq_system_snapshot", c_int, [POINTER(c_uint32), c_uint32, POINTER(c_uint32), POINTER(POINTER(c_uint64))]),
     ("sq_system_key_words", c_int, [POINTER(c_uint32)]),
     ("sq_system_set_register_type", c_int, [c_uint32, c_uint32]),
     ("sq_state_create", c_int, [c_uint64, POINTER(c_void_p)]),

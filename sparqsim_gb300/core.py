@@ -14,7 +14,8 @@ from typing import Iterable, Union
 
 import numpy as np
 
-from ._native import SqCond, call, lib
+from ._native import (COND_ALL_ONES, COND_BIT, COND_NONZERO, COND_VALUE, SQ_MAX_CONDITIONS, SQ_MAX_REGISTERS, SqCond,
+                      call, lib)
 
 RegRef = Union[str, int]
 
@@ -50,6 +51,7 @@ class System:
     def clear() -> None:
         call("sq_system_clear")
         System._names = []
+        System._by_name.clear()
 
     @staticmethod
     def add_register(name: str, type_: StateStorageType, size: int) -> int:
@@ -63,6 +65,7 @@ class System:
         while len(System._names) <= rid:
             System._names.append(None)
         System._names[rid] = name
+        System._by_name.clear()
 
     @staticmethod
     def add_register_synchronous(name: str, type_: StateStorageType, size: int, state: "SparseState") -> int:
@@ -79,22 +82,55 @@ class System:
     def remove_register_synchronous(reg: RegRef, state: "SparseState") -> None:
         call("sq_remove_register_sync", state._h, System.resolve(reg))
 
+    # Copy of the register table (five words per id, sq_system_snapshot), read
+    # again when the engine's change counter has moved: operators look several
+    # registers up by name each, and a call into the library per lookup was a
+    # third of a small walk step's time.
+    _rows: list = []
+    _by_name: dict = {}  # names looked up since the last change
+    _seen = 0
+    _changes = None
+    _buf = None
+
+    @staticmethod
+    def _table() -> list:
+        c = System._changes
+        if c is None or c.value != System._seen:
+            System._refresh()
+        return System._rows
+
+    @staticmethod
+    def _refresh() -> None:
+        if System._buf is None:
+            System._buf = (c_uint32 * (5 * SQ_MAX_REGISTERS))()
+        n, p = c_uint32(), ctypes.POINTER(c_uint64)()
+        call("sq_system_snapshot", System._buf, len(System._buf) // 5, byref(n), byref(p))
+        System._changes = p.contents
+        System._rows, System._seen = System._buf[:5 * n.value], p.contents.value
+        System._by_name.clear()
+
     @staticmethod
     def _info(rid: int):
-        t, w, a, wd, sh = (c_uint32(), c_uint32(), c_uint32(), c_uint32(), c_uint32())
-        call("sq_system_register_info", int(rid), byref(t), byref(w), byref(a), byref(wd), byref(sh))
-        return t.value, w.value, bool(a.value), wd.value, sh.value
+        rid = int(rid)
+        rows = System._table()
+        if not 0 <= 5 * rid < len(rows):
+            call("sq_system_register_info", rid, None, None, None, None, None)  # raises: register not found
+        t, w, a, wd, sh = rows[5 * rid:5 * rid + 5]
+        return t, w, bool(a), wd, sh
 
     @staticmethod
     def register_count() -> int:
-        n = c_uint32()
-        call("sq_system_register_count", byref(n))
-        return n.value
+        return len(System._table()) // 5
 
     @staticmethod
     def get_id(name: str) -> int:
-        for rid in range(min(len(System._names), System.register_count()) - 1, -1, -1):
-            if System._names[rid] == name and System._info(rid)[2]:
+        rows, names = System._table(), System._names
+        rid = System._by_name.get(name)
+        if rid is not None:
+            return rid
+        for rid in range(min(len(names), len(rows) // 5) - 1, -1, -1):
+            if names[rid] == name and rows[5 * rid + 2]:
+                System._by_name[name] = rid
                 return rid
         raise ValueError(f"Register not found: {name!r}")
 
@@ -369,6 +405,11 @@ class Controllable:
         self.condition_variable_by_bit = []
         self.condition_variable_by_value = []
 
+    def __copy__(self):
+        o = object.__new__(type(self))
+        o.__dict__.update(self.__dict__)
+        return o
+
     @staticmethod
     def _ids(conds) -> list:
         if isinstance(conds, (str, int, np.integer)):
@@ -420,8 +461,9 @@ class Controllable:
                     or self.condition_variable_by_bit or self.condition_variable_by_value)
 
     def _cond(self) -> SqCond:
-        from ._native import COND_ALL_ONES, COND_BIT, COND_NONZERO, COND_VALUE, SQ_MAX_CONDITIONS
         c = SqCond()
+        if not self.has_condition():
+            return c
         items = ([(COND_NONZERO, r, 0) for r in self.condition_variable_nonzeros]
                  + [(COND_ALL_ONES, r, 0) for r in self.condition_variable_all_ones]
                  + [(COND_BIT, r, p) for r, p in self.condition_variable_by_bit]

@@ -159,8 +159,12 @@ int sq_get_stream(void** s) {
 }
 
 // ------------------------------------------------------------------ registers
+// Counts the calls that may have changed the register table.
+static uint64_t g_table_changes = 1;
+
 int sq_system_clear(void) {
     SQ_API_BEGIN
+    ++g_table_changes;
     // the default prune threshold is a setting of its own, kept across a
     // clear as the reference's global clearzero_default_eps
     // (system_operations.h:577) is
@@ -173,6 +177,7 @@ int sq_system_clear(void) {
 
 int sq_system_add_register(uint32_t type, uint32_t width, uint32_t* id_out) {
     SQ_API_BEGIN
+    ++g_table_changes;
     need(id_out != nullptr, "null pointer");
     *id_out = regtable().add(type, width);
     SQ_API_END
@@ -180,6 +185,7 @@ int sq_system_add_register(uint32_t type, uint32_t width, uint32_t* id_out) {
 
 int sq_system_remove_register(uint32_t id) {
     SQ_API_BEGIN
+    ++g_table_changes;
     regtable().remove(id);
     SQ_API_END
 }
@@ -205,6 +211,20 @@ int sq_system_register_count(uint32_t* n) {
     SQ_API_END
 }
 
+int sq_system_snapshot(uint32_t* rows, uint32_t max_regs, uint32_t* n, const uint64_t** changes) {
+    SQ_API_BEGIN
+    need(n != nullptr && (rows != nullptr || max_regs == 0), "null pointer");
+    const RegTable& t = regtable();
+    *n = (uint32_t)t.regs.size();
+    for (uint32_t i = 0; i < *n && i < max_regs; ++i) {
+        const RegEntry& r = t.regs[i];
+        const uint32_t row[5] = {r.type, r.width, r.active ? 1u : 0u, r.word, r.shift};
+        std::copy(row, row + 5, rows + 5 * (size_t)i);
+    }
+    if (changes) *changes = &g_table_changes;
+    SQ_API_END
+}
+
 int sq_system_key_words(uint32_t* k) {
     SQ_API_BEGIN
     need(k != nullptr, "null pointer");
@@ -214,6 +234,7 @@ int sq_system_key_words(uint32_t* k) {
 
 int sq_system_set_register_type(uint32_t id, uint32_t type) {
     SQ_API_BEGIN
+    ++g_table_changes;
     need(type <= SQ_RATIONAL, "bad register type");
     (void)regtable().at(id);
     regtable().regs[id].type = type;
@@ -1484,6 +1505,7 @@ int sq_add_systems(sq_state* dst, const sq_state* src, double coef) {
 
 int sq_add_register_sync(sq_state* st, uint32_t type, uint32_t width, uint32_t* id_out) {
     SQ_API_BEGIN
+    ++g_table_changes;
     need(id_out != nullptr, "null pointer");
     State& s = S(st);
     drop_groups(s);
@@ -1495,6 +1517,7 @@ int sq_add_register_sync(sq_state* st, uint32_t type, uint32_t width, uint32_t* 
 
 int sq_add_register_with_hadamard(sq_state* st, uint32_t type, uint32_t width, uint32_t* id_out) {
     SQ_API_BEGIN
+    ++g_table_changes;
     need(id_out != nullptr, "null pointer");
     State& s = S(st);
     drop_groups(s);
@@ -1520,6 +1543,7 @@ int sq_add_register_with_hadamard(sq_state* st, uint32_t type, uint32_t width, u
 
 int sq_remove_register_sync(sq_state* st, uint32_t id) {
     SQ_API_BEGIN
+    ++g_table_changes;
     State& s = S(st);
     drop_groups(s);
     Field f = regtable().field(id);
@@ -1530,6 +1554,7 @@ int sq_remove_register_sync(sq_state* st, uint32_t id) {
 
 int sq_split_register(sq_state* st, uint32_t first, uint32_t second_size, uint32_t* second_out) {
     SQ_API_BEGIN
+    ++g_table_changes;
     need(second_out != nullptr, "null pointer");
     State& s = S(st);
     drop_groups(s);
@@ -1554,6 +1579,7 @@ int sq_split_register(sq_state* st, uint32_t first, uint32_t second_size, uint32
 
 int sq_combine_register(sq_state* st, uint32_t first, uint32_t second) {
     SQ_API_BEGIN
+    ++g_table_changes;
     State& s = S(st);
     drop_groups(s);
     RegTable& t = regtable();
