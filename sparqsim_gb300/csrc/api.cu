@@ -68,6 +68,10 @@ static State& S(sq_state* st) {
     need(st != nullptr, "null state");
     if (capturing() && st != g_capture_state) fail(SQ_ERR_INVALID, "capture: operators on another state");
     State& s = st->s;
+    // an operator may write any active register: only inactive bits stay known
+    uint64_t active[SQ_KMAX];
+    regtable().active_mask(active);
+    for (uint32_t w = 0; w < SQ_KMAX; ++w) s.zeroed[w] &= w < regtable().k ? ~active[w] : 0ull;  // words past k go stale
     if (s.d2h_pending) {
         SQ_CUDA(cudaStreamWaitEvent(stream(), s.d2h_done, 0));
         s.d2h_pending = false;
@@ -345,6 +349,8 @@ int sq_state_copy(sq_state* dst, const sq_state* src) {
     }
     SQ_CUDA(cudaMemcpyAsync(d.live.amp, s.live.amp, s.n * 16, cudaMemcpyDeviceToDevice, stream()));
     d.n = s.n;
+    std::copy(s.zeroed, s.zeroed + SQ_KMAX, d.zeroed);
+    for (uint32_t w = k; w < SQ_KMAX; ++w) d.zeroed[w] = 0;  // words that were not copied
     SQ_API_END
 }
 
@@ -410,6 +416,7 @@ int sq_state_upload_packed(sq_state* st, uint64_t n, const uint64_t* keys, const
     need(n == 0 || (keys != nullptr && amps != nullptr), "null pointer");
     const uint32_t k = regtable().k;
     ensure_buffers(s.live, std::max<uint64_t>(n, 1), k, 0);
+    memset(s.zeroed, 0, sizeof(s.zeroed));  // the caller's words, whatever they hold
     std::vector<CopyJob> jobs;
     for (uint32_t w = 0; w < k; ++w) jobs.push_back({s.live.keys[w], keys + (size_t)w * n, (size_t)n * 8});
     jobs.push_back({s.live.amp, amps, (size_t)n * 16});
@@ -690,6 +697,7 @@ int sq_state_device_arrays(sq_state* st, uint64_t** key_words, uint32_t* k, doub
     SQ_API_BEGIN
     State& s = S(st);
     drop_groups(s);  // the caller may write the arrays
+    memset(s.zeroed, 0, sizeof(s.zeroed));
     sync_words(s);
     if (key_words)
         for (uint32_t w = 0; w < regtable().k; ++w) key_words[w] = s.live.keys[w];

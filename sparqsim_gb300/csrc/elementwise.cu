@@ -1117,6 +1117,8 @@ void zero_field(State& s, Field f) {
     sync_words(s);
     if (s.n == 0 || f.width == 0) return;
     const uint64_t keep = ~(wmask(f.width) << f.shift);
+    if (!(~keep & ~s.zeroed[f.word])) return;  // cleared when its last register was removed
+    s.zeroed[f.word] |= ~keep;
     prof_begin("zero_field");
     zero_field_kernel<1><<<grid_for(s.n, 256), 256, 0, stream()>>>(s.live.keys[f.word], keep, s.n);
     prof_end((double)s.n * 16);

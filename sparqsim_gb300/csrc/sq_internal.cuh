@@ -213,6 +213,11 @@ struct State {
     Buffers live;
     Buffers spare;
     uint64_t n = 0;
+    // Bits of inactive registers known to be 0 in every entry: what zero_field
+    // has cleared and no register covers since. A register that gets such bits
+    // needs no clearing pass (drivers remove and add the same scratch registers
+    // tens of times per walk step).
+    uint64_t zeroed[SQ_KMAX] = {0};
     GroupCache groups;
     uint64_t swaps = 0;              // live/spare exchanges so far (graphs need an even number per sequence)
     cudaEvent_t d2h_done = nullptr;  // recorded when the last asynchronous download finished reading
