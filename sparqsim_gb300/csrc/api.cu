@@ -523,7 +523,8 @@ static uint64_t state_checksum(const State& s) {
 int sq_graph_record_begin(sq_state* st) {
     SQ_API_BEGIN
     need(replay().mode == RP_OFF, "graph: a record or capture is already open");
-    const State& s = S(st);
+    State& s = S(st);
+    settle_swap(s);
     g_record_state = st;
     g_record_swaps = s.swaps;
     g_record_cur = s.groups.cur;
@@ -555,6 +556,7 @@ int sq_graph_capture_begin(sq_state* st) {
     SQ_API_BEGIN
     need(replay().mode == RP_OFF, "graph: a record or capture is already open");
     State& s = S(st);
+    settle_swap(s);
     SQ_CUDA(cudaStreamSynchronize(stream()));
     need(state_checksum(s) == g_record_input_sum, "graph: the capture does not start from the recorded input");
     g_capture_pre = s;
@@ -624,6 +626,7 @@ int sq_graph_launch(sq_graph* g) {
         need(g->table_gens[i] != 0 && table_generation(g->tables[i].first) == g->table_gens[i],
              "graph: a table it reads has been destroyed");
     State& s = S(g->st);
+    settle_swap(s);
     need(same_layout(s, g->pre), "graph: the state's size or buffers differ from the captured ones");
     for (int i = 0; i < WS_COUNT_MAX; ++i)
         need(ws().p[i] == g->ws_p[i], "graph: the library's workspace has been reallocated");

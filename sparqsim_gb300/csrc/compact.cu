@@ -5,6 +5,7 @@
 // once, and writes the survivors once: N*16 + N_out*(8K+16) bytes, the
 // algorithmic minimum. Tile offsets come from a decoupled look-back, so the
 // kernel is a single pass and keeps the reference's remove_if order.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <limits>
@@ -25,10 +26,11 @@ struct LookbackWs {
 };
 
 // Layout of the look-back workspace: [counter (u32) | total (u64) | pad to 256 B | status[ntiles]].
+// One tile waits for none and takes no ticket: its words need no clearing.
 static LookbackWs lookback_ws(long long ntiles) {
     size_t bytes = 256 + (size_t)ntiles * 8;
     char* p = (char*)ws().get(WS_LOOKBACK, bytes);
-    SQ_CUDA(cudaMemsetAsync(p, 0, bytes, stream()));
+    if (ntiles > 1) SQ_CUDA(cudaMemsetAsync(p, 0, bytes, stream()));
     LookbackWs w;
     w.counter = (unsigned*)p;
     w.total = (unsigned long long*)(p + 8);
@@ -47,18 +49,50 @@ struct KeySelect {
     uint64_t lo, hi;
 };
 
+// Whether ClearZero has anything to drop. Every split prunes its outputs at the
+// same threshold, so the ClearZero calls that the walks make after them almost
+// never do: 16 bytes read per entry instead of 24 K + 48 (read, and written to
+// the other buffer). A CKS term's four calls at 2.6 M entries of six words:
+// 410 us of kernels in one pass, 60 when the check lets them be skipped.
+__global__ void __launch_bounds__(kCzBlock) prune_any_kernel(const double2* __restrict__ a, uint64_t n, double eps,
+                                                             unsigned* __restrict__ any) {
+    const uint64_t stride = (uint64_t)gridDim.x * kCzTile;
+    bool drop = false;
+    for (uint64_t b = (uint64_t)blockIdx.x * kCzTile; b < n; b += stride) {
+        double2 v[kCzItems];
+#pragma unroll
+        for (int j = 0; j < kCzItems; ++j) {
+            const uint64_t i = b + (uint64_t)j * kCzBlock + threadIdx.x;
+            v[j] = i < n ? a[i] : make_double2(__longlong_as_double(0x7ff0000000000000ll), 0.0);  // kept
+        }
+#pragma unroll
+        for (int j = 0; j < kCzItems; ++j) drop = drop || !sq_keep_amp(v[j].x, v[j].y, eps);
+    }
+    if (__syncthreads_or(drop) && threadIdx.x == 0) *any = 1u;
+}
+
+constexpr unsigned long long kCzUnchanged = 1ull << 63;
+
 // SEL = false: ClearZero (keep |a|^2 >= eps); SEL = true: keep the entries the
-// key selection accepts. Same single pass either way.
+// key selection accepts. Same single pass either way. any: prune_any's word
+// (null: compact whatever it would say); the number of survivors, or n |
+// kCzUnchanged when nothing was written, is posted to the host.
 template <int K, bool SEL>
 __global__ void __launch_bounds__(kCzBlock) clearzero_kernel(ConstKeyPtrs ik, const double2* __restrict__ ia,
                                                              KeyPtrs ok, double2* __restrict__ oa, uint64_t n,
                                                              double eps, LookbackWs lb, long long ntiles,
-                                                             unsigned* err, const __grid_constant__ KeySelect ks) {
+                                                             unsigned* err, const __grid_constant__ KeySelect ks,
+                                                             const unsigned* __restrict__ any,
+                                                             const __grid_constant__ MailSlot mail) {
     __shared__ unsigned s_tile;
     __shared__ unsigned s_cnt[kCzItems][kCzBlock / 32];
     __shared__ unsigned long long s_prefix;
     const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    if (tid == 0) s_tile = atomicAdd(lb.counter, 1u);
+    if (any && *any == 0u) {
+        if (blockIdx.x == 0 && tid == 0) mail_post(mail, n | kCzUnchanged);
+        return;
+    }
+    if (tid == 0) s_tile = ntiles == 1 ? 0u : atomicAdd(lb.counter, 1u);
     __syncthreads();
     const long long tile = s_tile;
     const uint64_t base = (uint64_t)tile * kCzTile;
@@ -104,7 +138,10 @@ __global__ void __launch_bounds__(kCzBlock) clearzero_kernel(ConstKeyPtrs ik, co
         unsigned long long pre = lb_warp_exclusive(lb.status, tile, total, err);
         if (lane == 0) {
             s_prefix = pre;
-            if (tile == ntiles - 1) *lb.total = pre + total;
+            if (tile == ntiles - 1) {
+                *lb.total = pre + total;
+                mail_post(mail, pre + total);
+            }
         }
     }
     __syncthreads();
@@ -123,7 +160,7 @@ __global__ void __launch_bounds__(kCzBlock) clearzero_kernel(ConstKeyPtrs ik, co
 
 template <int K, bool SEL = false>
 static void launch_cz(const Buffers& in, Buffers& out, uint64_t n, double eps, LookbackWs lb, long long nt,
-                      const KeySelect* ks = nullptr) {
+                      const KeySelect* ks = nullptr, const unsigned* any = nullptr, const MailSlot& mail = MailSlot()) {
     ConstKeyPtrs ik;
     KeyPtrs okp;
     for (int w = 0; w < SQ_KMAX; ++w) {
@@ -134,7 +171,7 @@ static void launch_cz(const Buffers& in, Buffers& out, uint64_t n, double eps, L
     memset(&none, 0, sizeof(none));
     prof_begin(SEL ? "select_entries" : "clearzero");
     clearzero_kernel<K, SEL><<<(unsigned)nt, kCzBlock, 0, stream()>>>(ik, in.amp, okp, out.amp, n, eps, lb, nt,
-                                                                    device_error_word(), ks ? *ks : none);
+                                                                    device_error_word(), ks ? *ks : none, any, mail);
     prof_end((double)n * 16);  // every amplitude read; survivors added below
     SQ_CUDA(cudaGetLastError());
 }
@@ -202,7 +239,7 @@ void selftest_wait_timeout(unsigned polls) {
     KeySelect none;
     memset(&none, 0, sizeof(none));
     clearzero_kernel<1, false><<<1, kCzBlock, 0, stream()>>>(ik, ain, okp, aout, n, 1e-14, lb, 2,
-                                                              device_error_word(), none);
+                                                              device_error_word(), none, nullptr, MailSlot());
     count_launch();
     const cudaError_t le = cudaGetLastError();
     set_wait_limit(prev);  // synchronizes: the block has finished
@@ -211,25 +248,34 @@ void selftest_wait_timeout(unsigned polls) {
 }
 
 // Compacts `in` (n entries) into `out`, returns the survivor count. `out`
-// must already hold n entries of capacity.
-uint64_t compact_nonzero(const Buffers& in, Buffers& out, uint64_t n, double eps, uint32_t k) {
+// must already hold n entries of capacity. With `check`, nothing is written
+// and kCzUnchanged is set when every entry survives.
+uint64_t compact_nonzero(const Buffers& in, Buffers& out, uint64_t n, double eps, uint32_t k, bool check) {
     if (n == 0) return 0;
     const long long nt = (long long)((n + kCzTile - 1) / kCzTile);
     LookbackWs lb = lookback_ws(nt);
+    unsigned* any = nullptr;
+    if (check) {
+        any = (unsigned*)(lb.total + 1);
+        prof_begin("prune_check");
+        prune_any_kernel<<<grid_for(n, kCzTile, 8), kCzBlock, 0, stream()>>>(in.amp, n, eps, any);
+        prof_end((double)n * 16);
+    }
+    const MailSlot mail = mail_slot();
     switch (k) {
-        case 1: launch_cz<1>(in, out, n, eps, lb, nt); break;
-        case 2: launch_cz<2>(in, out, n, eps, lb, nt); break;
-        case 3: launch_cz<3>(in, out, n, eps, lb, nt); break;
-        case 4: launch_cz<4>(in, out, n, eps, lb, nt); break;
-        case 5: launch_cz<5>(in, out, n, eps, lb, nt); break;
-        case 6: launch_cz<6>(in, out, n, eps, lb, nt); break;
-        case 7: launch_cz<7>(in, out, n, eps, lb, nt); break;
-        default: launch_cz<8>(in, out, n, eps, lb, nt); break;
+        case 1: launch_cz<1>(in, out, n, eps, lb, nt, nullptr, any, mail); break;
+        case 2: launch_cz<2>(in, out, n, eps, lb, nt, nullptr, any, mail); break;
+        case 3: launch_cz<3>(in, out, n, eps, lb, nt, nullptr, any, mail); break;
+        case 4: launch_cz<4>(in, out, n, eps, lb, nt, nullptr, any, mail); break;
+        case 5: launch_cz<5>(in, out, n, eps, lb, nt, nullptr, any, mail); break;
+        case 6: launch_cz<6>(in, out, n, eps, lb, nt, nullptr, any, mail); break;
+        case 7: launch_cz<7>(in, out, n, eps, lb, nt, nullptr, any, mail); break;
+        default: launch_cz<8>(in, out, n, eps, lb, nt, nullptr, any, mail); break;
     }
     unsigned long long total = 0;
-    host_read(&total, lb.total, 8);
-    check_device_error();  // synchronizes
-    prof_add_bytes_last((double)total * (16.0 * k + 16));  // survivors: keys read + keys and amp written
+    mail_read(mail, &total, lb.total, 8);
+    check_device_error();
+    if (!(total & kCzUnchanged)) prof_add_bytes_last((double)total * (16.0 * k + 16));  // survivors: keys read + keys and amp written
     return total;
 }
 
@@ -392,29 +438,81 @@ void clear_zero(State& s, double eps) {
     if (s.n == 0) return;
     const uint32_t k = regtable().k;
     ensure_buffers(s.spare, s.n, k, 0);
-    uint64_t m = compact_nonzero(s.live, s.spare, s.n, eps, k);
+    // a recorded or captured ClearZero always compacts, as its sequence counts on the buffers' exchange
+    const bool check = s.n > (uint64_t)kCzTile && replay().mode == RP_OFF;
+    const uint64_t m = compact_nonzero(s.live, s.spare, s.n, eps, k, check);
+    if (m & kCzUnchanged) {
+        s.owes_swap = !s.owes_swap;
+        return;
+    }
     swap_live_spare(s);
     s.n = m;
 }
 
+void settle_swap(State& s) {
+    if (!s.owes_swap) return;
+    const uint32_t k = regtable().k;
+    sync_words(s);
+    ensure_buffers(s.spare, s.n, k, 0);
+    for (uint32_t w = 0; w < k; ++w)
+        SQ_CUDA(cudaMemcpyAsync(s.spare.keys[w], s.live.keys[w], s.n * 8, cudaMemcpyDeviceToDevice, stream()));
+    SQ_CUDA(cudaMemcpyAsync(s.spare.amp, s.live.amp, s.n * 16, cudaMemcpyDeviceToDevice, stream()));
+    swap_live_spare(s);
+    s.owes_swap = false;
+}
+
 // ------------------------------------------------------------------ norm
 
-__global__ void __launch_bounds__(kRedBlock) norm_partial_kernel(const double2* __restrict__ a, uint64_t n,
-                                                                 double* __restrict__ partial) {
+// Sum of |a|^2: per-thread sums in entry order, a tree per CTA, and the CTA that
+// finishes last sums the CTAs' results in their order (norm_final's), so the
+// value does not depend on timing; it posts it to the host. Two fused
+// multiply-adds per entry: the FP64 pipe (2 lanes per SM and clock) was the
+// bound with two products and two sums (2.6 M entries: 20 us, 13 here).
+// ticket: zero between launches.
+__global__ void __launch_bounds__(kRedBlock) norm_kernel(const double2* __restrict__ a, uint64_t n,
+                                                         double* __restrict__ partial, unsigned* ticket,
+                                                         double* __restrict__ out,
+                                                         const __grid_constant__ MailSlot mail) {
     __shared__ double s[kRedBlock];
+    __shared__ bool s_last;
     double acc = 0.0;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (; i + 3 * stride < n; i += 4 * stride) {
+        double2 v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = a[i + q * stride];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc = __fma_rn(v[q].x, v[q].x, __fma_rn(v[q].y, v[q].y, acc));
+    }
+    for (; i < n; i += stride) {
         const double2 v = a[i];
-        acc += v.x * v.x + v.y * v.y;
+        acc = __fma_rn(v.x, v.x, __fma_rn(v.y, v.y, acc));
     }
-    s[threadIdx.x] = acc;
-    __syncthreads();
-    for (int o = kRedBlock / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
+    for (int round = 0; round < 2; ++round) {
+        s[threadIdx.x] = acc;
         __syncthreads();
+        for (int o = kRedBlock / 2; o > 0; o >>= 1) {
+            if ((int)threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
+            __syncthreads();
+        }
+        if (round == 1) break;
+        if (threadIdx.x == 0) {
+            partial[blockIdx.x] = s[0];
+            __threadfence();
+            s_last = atomicAdd(ticket, 1u) == gridDim.x - 1u;
+        }
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+        acc = 0.0;
+        for (int j = threadIdx.x; j < (int)gridDim.x; j += kRedBlock) acc += __ldcg(partial + j);
     }
-    if (threadIdx.x == 0) partial[blockIdx.x] = s[0];
+    if (threadIdx.x == 0) {
+        *out = s[0];
+        *ticket = 0u;
+        mail_post(mail, (unsigned long long)__double_as_longlong(s[0]));
+    }
 }
 
 __global__ void __launch_bounds__(kRedBlock) norm_final_kernel(const double* __restrict__ partial, int m,
@@ -433,17 +531,21 @@ __global__ void __launch_bounds__(kRedBlock) norm_final_kernel(const double* __r
 
 double norm_sq(const State& s) {
     if (s.n == 0) return 0.0;
-    const int g = num_sms() * 4;
-    double* part = (double*)ws().get(WS_REDUCE, (size_t)(g + 1) * 8);
-    prof_begin("norm_partial");
-    norm_partial_kernel<<<g, kRedBlock, 0, stream()>>>(s.live.amp, s.n, part);
+    // CTAs past the entries would add zeros
+    const int g = (int)std::min<uint64_t>((uint64_t)num_sms() * 4, (s.n + kRedBlock - 1) / kRedBlock);
+    double* part = (double*)ws().get(WS_REDUCE, (size_t)(num_sms() * 4 + 1) * 8);
+    static unsigned* ticket = nullptr;
+    if (!ticket) {
+        ticket = (unsigned*)dev_alloc(16);
+        SQ_CUDA(cudaMemsetAsync(ticket, 0, 16, stream()));
+    }
+    const MailSlot mail = mail_slot();
+    prof_begin("norm");
+    norm_kernel<<<g, kRedBlock, 0, stream()>>>(s.live.amp, s.n, part, ticket, part + g, mail);
     prof_end((double)s.n * 16);
-    prof_begin("norm_final");
-    norm_final_kernel<<<1, kRedBlock, 0, stream()>>>(part, g, part + g);
-    prof_end((double)g * 8);
     SQ_CUDA(cudaGetLastError());
     double r = 0;
-    host_read(&r, part + g, 8);
+    mail_read(mail, &r, part + g, 8);
     return r;
 }
 
@@ -500,7 +602,7 @@ static void launch_cz_noalloc(const uint64_t* const* keys_in, const double* amps
     memset(&none, 0, sizeof(none));
     clearzero_kernel<K, false><<<(unsigned)nt, kCzBlock, 0, s>>>(ik, (const double2*)amps_in, okp,
                                                                  (double2*)amps_out, n, eps, lb, nt,
-                                                                 (unsigned*)(scratch + 2), none);
+                                                                 (unsigned*)(scratch + 2), none, nullptr, MailSlot());
     count_launch();
 }
 

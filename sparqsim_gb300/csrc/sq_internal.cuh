@@ -219,6 +219,10 @@ struct State {
     // tens of times per walk step).
     uint64_t zeroed[SQ_KMAX] = {0};
     GroupCache groups;
+    // A ClearZero that drops nothing leaves the entries where they are instead
+    // of exchanging the buffers. Graphs are bound to the buffers' roles, which
+    // must depend on the operators alone: settle_swap makes up for it there.
+    bool owes_swap = false;
     uint64_t swaps = 0;              // live/spare exchanges so far (graphs need an even number per sequence)
     cudaEvent_t d2h_done = nullptr;  // recorded when the last asynchronous download finished reading
     bool d2h_pending = false;        // the library stream has not been made to wait for it yet
@@ -393,6 +397,7 @@ inline unsigned grid_for(uint64_t n, int block, int per_sm = 8) {
 struct DInstr;
 void run_program(State& s, const sq_instr* prog, uint32_t n);
 void clear_zero(State& s, double eps);
+void settle_swap(State& s);
 double norm_sq(const State& s);
 void scale_amp(State& s, double k);
 void add_systems(State& dst, const State& src, double coef);
