@@ -266,13 +266,7 @@ int sq_state_create(uint64_t capacity, sq_state** out) {
     sq_state* st = new sq_state();
     try {
         ensure_buffers(st->s.live, capacity ? capacity : 1, regtable().k, 0);
-        // one entry |0...0>, amplitude 1
-        double2 one = make_double2(1.0, 0.0);
-        SQ_CUDA(cudaMemcpyAsync(st->s.live.amp, &one, sizeof(one), cudaMemcpyHostToDevice, stream()));
-        for (uint32_t w = 0; w < st->s.live.kalloc; ++w)
-            SQ_CUDA(cudaMemsetAsync(st->s.live.keys[w], 0, 8, stream()));
-        SQ_CUDA(cudaStreamSynchronize(stream()));
-        st->s.n = 1;
+        ground_state(st->s);
     } catch (...) {
         free_buffers(st->s.live);
         delete st;
@@ -326,11 +320,8 @@ int sq_state_reset(sq_state* st) {
     drop_groups(s);
     sync_words(s);
     ensure_buffers(s.live, 1, regtable().k, 0);
-    double2 one = make_double2(1.0, 0.0);
-    SQ_CUDA(cudaMemcpyAsync(s.live.amp, &one, sizeof(one), cudaMemcpyHostToDevice, stream()));
-    for (uint32_t w = 0; w < s.live.kalloc; ++w) SQ_CUDA(cudaMemsetAsync(s.live.keys[w], 0, 8, stream()));
-    SQ_CUDA(cudaStreamSynchronize(stream()));
-    s.n = 1;
+    if (capturing()) fail(SQ_ERR_CUDA, "capture: a state would be reset");
+    ground_state(s);
     SQ_API_END
 }
 
@@ -1243,6 +1234,9 @@ int sq_rot_general_unitary(sq_state* st, uint32_t reg, const double* mat, uint64
     g.target = f;
     g.umat = dev;
     g.udag = dag ? 1 : 0;
+    g.ureal = 1;
+    for (uint64_t i = 0; i < dim * dim; ++i)
+        if (mat[2 * i + 1] != 0.0) g.ureal = 0;
     g.cond = resolve_cond(cond);
     g.eps = cz_eps();
     group_transform(S(st), g);

@@ -433,6 +433,7 @@ struct EmitArgs {
     const double2* mtable;     // CondRot_General_Bool: 4 matrix elements per input value
     const double2* umat;       // Rot_GeneralUnitary: S x S row-major
     int udag;                  // Rot_GeneralUnitary: apply the conjugate transpose
+    int ureal;                 // umat has no imaginary parts
     Field varw;                // batched Hadamard: each group's digit count is this field of its key
     const unsigned long long* rstart;  // cached group ranges (access mode 2)
     const unsigned* rcnt;
@@ -1273,12 +1274,24 @@ __global__ void __launch_bounds__(256) emit_small_kernel(const __grid_constant__
                     // An empty slot's terms are +-0 and leave every nonzero sum as it is (an all-zero
                     // output is pruned), so column j is skipped when no lane of the warp holds slot j:
                     // FP64 is the limit of this kernel, and partly filled groups are common.
+                    // A real matrix (the tridiagonal encoding's preparation) needs half of it: the
+                    // products with its zero parts leave finite sums as they are (zero signs aside).
                     double2 r[S];
+                    bool real = a.ureal != 0;
 #pragma unroll
-                    for (unsigned c = 0; c < S; ++c) r[c] = make_double2(0.0, 0.0);
+                    for (unsigned c = 0; c < S; ++c) {
+                        r[c] = make_double2(0.0, 0.0);
+                        real = real && finite2(v[c]);
+                    }
 #pragma unroll
                     for (unsigned j = 0; j < S; ++j) {
                         if (!__any_sync(__activemask(), (filled >> j) & 1u)) continue;
+                        if (real) {
+#pragma unroll
+                            for (unsigned c = 0; c < S; ++c)
+                                r[c] = cadd(r[c], cscale(v[j], a.umat[a.udag ? j * S + c : c * S + j].x));
+                            continue;
+                        }
 #pragma unroll
                         for (unsigned c = 0; c < S; ++c) {
                             const double2 mij = a.udag ? make_double2(a.umat[j * S + c].x, -a.umat[j * S + c].y)
@@ -2618,7 +2631,8 @@ __global__ void __launch_bounds__(1024) group_small_kernel(const __grid_constant
                                                            unsigned max_digits, unsigned* __restrict__ counts,
                                                            unsigned* __restrict__ seg, unsigned* __restrict__ ghead,
                                                            unsigned* __restrict__ btgt, double2* __restrict__ bamp,
-                                                           unsigned* __restrict__ pass_list, unsigned* err) {
+                                                           unsigned* __restrict__ pass_list, unsigned* err,
+                                                           const __grid_constant__ MailSlot mail) {
     constexpr unsigned kSmallBatch = small_batch<K>();
     extern __shared__ unsigned s_tab[];  // cap slots | cap counts
     unsigned* table = s_tab;
@@ -2707,6 +2721,7 @@ __global__ void __launch_bounds__(1024) group_small_kernel(const __grid_constant
             counts[0] = n;
             counts[1] = 0u;
             seg[n] = n;
+            mail_post(mail, n);
         }
         return;
     }
@@ -2761,6 +2776,7 @@ __global__ void __launch_bounds__(1024) group_small_kernel(const __grid_constant
         counts[0] = s_scan[31][0];
         counts[1] = s_F;
         seg[s_scan[31][0]] = s_scan[31][1];
+        mail_post(mail, (unsigned long long)s_scan[31][0] | ((unsigned long long)s_F << 32));
     }
     __syncthreads();
     // members, contiguous per group
@@ -3091,16 +3107,17 @@ static Grouping group_by_hash(State& s, const GroupSpec& gs, uint64_t* dg, uint6
                                          (int)(2 * 2 * kSmallGroupMax * 4)));
             smem_set = true;
         }
+        const MailSlot mail = mail_slot();
         prof_begin("group_small");
         group_small_kernel<K><<<1, 1024, 2 * cap * 4, st>>>(
             ik, dg, gs.cond, s.live.amp, (unsigned)N, cap, gs.target, gs.varw, gs.target.width, (unsigned*)base,
             (unsigned*)(base + o_seg), (unsigned*)(base + o_head), (unsigned*)(base + o_btgt),
-            (double2*)(base + o_bamp), (unsigned*)(base + o_pass), device_error_word());
+            (double2*)(base + o_bamp), (unsigned*)(base + o_pass), device_error_word(), mail);
         prof_end((double)N * (8.0 * K + 16) * 2);
         SQ_CUDA(cudaGetLastError());
         unsigned gc[2] = {0, 0};
-        host_read(gc, base, 8);
-        check_device_error();  // synchronizes
+        mail_read(mail, gc, base, 8);
+        check_device_error();
         Grouping out;
         out.G = gc[0];
         out.F = gc[1];
@@ -3997,7 +4014,9 @@ static void run_group(State& s, const GroupSpec& gs) {
     h2d_small(dg, gmask, SQ_KMAX * 8);
 
     // the merge sums runs in order, so it keeps the (stable) sort; the
-    // transforms are order-independent and default to the hash grouping
+    // transforms are order-independent and default to the hash grouping, small
+    // states as well: one CTA groups 1024 entries in 12 us, where the sort
+    // takes six launches and 46 us of kernels
     int strat = get_group_strategy();
     uint64_t tune_key = 0;
     const bool tuned = strat == 3 && gs.mode != GM_MERGE && !gs.varw.width && N >= 4096;
@@ -4008,7 +4027,7 @@ static void run_group(State& s, const GroupSpec& gs) {
     } else if (strat == 3) {
         strat = 0;
     }
-    const bool use_hash = gs.varw.width || (gs.mode != GM_MERGE && (strat == 2 || (strat == 0 && N >= 4096)));
+    const bool use_hash = gs.varw.width || (gs.mode != GM_MERGE && strat != 1);
     struct TuneTimer {
         bool on;
         uint64_t key;
@@ -4081,6 +4100,7 @@ static void run_group(State& s, const GroupSpec& gs) {
     ea.real = real_matrix(gs);
     ea.umat = gs.umat;
     ea.udag = gs.udag;
+    ea.ureal = gs.ureal;
     ea.varw = gs.varw;
     ea.fix = get_fwht_arithmetic() == SQ_ARITH_EXACT_SUM ? 1 : 0;
     if (reuse) {

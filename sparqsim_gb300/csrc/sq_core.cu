@@ -829,6 +829,20 @@ void ensure_buffers(Buffers& b, uint64_t cap, uint32_t k, uint64_t keep) {
     b = nb;
 }
 
+__global__ void ground_state_kernel(KeyPtrs keys, unsigned words, double2* amp) {
+    if (threadIdx.x < words) keys.w[threadIdx.x][0] = 0ull;
+    if (threadIdx.x == 0) *amp = make_double2(1.0, 0.0);
+}
+
+void ground_state(State& s) {
+    KeyPtrs kp;
+    for (int w = 0; w < SQ_KMAX; ++w) kp.w[w] = s.live.keys[w];
+    ground_state_kernel<<<1, SQ_KMAX, 0, stream()>>>(kp, s.live.kalloc, s.live.amp);
+    SQ_CUDA(cudaGetLastError());
+    count_launch();
+    s.n = 1;
+}
+
 void sync_words(State& s) {
     uint32_t k = regtable().k;
     if (s.live.kalloc < k) ensure_buffers(s.live, s.live.cap, k, s.n);

@@ -351,6 +351,8 @@ void ensure_buffers(Buffers& b, uint64_t cap, uint32_t k, uint64_t keep);
 // Make the state's live buffers hold K = regtable().k words.
 void sync_words(State& s);
 void free_buffers(Buffers& b);
+// The single entry |0...0>, amplitude 1, in the live buffers (one launch; nothing waits for it).
+void ground_state(State& s);
 void swap_live_spare(State& s);
 
 // Workspace (grow-only device scratch shared by all operators).
@@ -423,6 +425,7 @@ struct GroupSpec {
     const double2* mtable;  // device: CondRot_General_Bool matrices (4 per input value)
     const double2* umat;    // device: Rot_GeneralUnitary matrix
     int udag;
+    int ureal;              // umat has no imaginary parts
     Field varw;             // batched Hadamard: register holding each entry's digit count (width 0: unused)
     int unscaled;           // Hadamard singleton fan-out without the 2^(-n/2) factor (AddRegisterWithHadamard)
 };
