@@ -3463,6 +3463,172 @@ __global__ void __launch_bounds__(256) pair_lone_kernel(const __grid_constant__ 
     }
 }
 
+// Where the registers span few enough bits of a one-word key, the bits
+// themselves index the table: one plain store per entry puts it in its slot
+// and one load finds its partner's, with no hash, no probing, no
+// compare-and-swap and no clear (a slot that nobody wrote in this split may
+// hold anything: it is believed only if it names an entry whose key and
+// conditions are the partner's, and then that entry did write it). Lone
+// entries are known at once, so there is no pass over them either. A dense
+// 2^21-entry split: 65 us of kernels (16 scatter, 49 pairs) against 125.
+struct PairDirect {
+    unsigned* slot;
+    unsigned lo;           // lowest register bit
+    unsigned long long mask;  // the registers' bits, shifted down by lo
+    unsigned* flags;       // as in PairTable; bit 2: a key has bits outside the registers
+};
+constexpr unsigned kPairStray = 4u;
+
+// Every passing entry into its slot. Of entries with the same key (uploaded
+// so) the last to write owns it; the others stay lone.
+template <int K>
+__global__ void __launch_bounds__(256) pair_scatter_kernel(ConstKeyPtrs keys, uint64_t n,
+                                                           const __grid_constant__ DCondSet cond, Field tgt,
+                                                           PairDirect d) {
+    static_assert(K == 1, "one key word");
+    const uint64_t stride = (uint64_t)gridDim.x * 1024u;
+    unsigned f = 0;
+    for (uint64_t b = (uint64_t)blockIdx.x * 1024u; b < n; b += stride) {
+        uint64_t k[4][1];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint64_t i = b + (uint64_t)q * 256u + threadIdx.x;
+            k[q][0] = i < n ? keys.w[0][i] : 0ull;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint64_t i = b + (uint64_t)q * 256u + threadIdx.x;
+            if (i >= n) continue;
+            if (k[q][0] & ~(d.mask << d.lo)) f |= kPairStray;
+            if (!cond_ok<1>(k[q], cond)) continue;
+            f |= fget<1>(k[q], tgt) ? 2u : 1u;
+            d.slot[(k[q][0] >> d.lo) & d.mask] = (unsigned)i;
+        }
+    }
+    f = __reduce_or_sync(0xffffffffu, f);
+    if ((threadIdx.x & 31u) == 0u && (f & ~*reinterpret_cast<volatile unsigned*>(d.flags))) atomicOr(d.flags, f);
+}
+
+// Pairs (by their member with target bit 0), lone entries and copies. A CTA
+// lists what its entries have to compute in shared memory, in entry order,
+// and its threads take the list's items, so that no FP64 lane idles for an
+// entry whose partner does the work. ITEMS entries per thread keep their
+// lookups in flight together. Bound by the chain key, slot, partner's key,
+// amplitudes (36 % issue, FP64 pipe 23 %), so CTAs in flight count: four
+// entries per thread at 64 registers 56 us, two at 40 registers 49 (2^21
+// entries); writing each target value's outputs as a run of its own: 56.
+template <int K, int ITEMS>
+__global__ void __launch_bounds__(256, 6) pair_direct_kernel(const __grid_constant__ EmitArgs a, uint64_t n,
+                                                          const __grid_constant__ DCondSet cond, PairDirect d) {
+    static_assert(K == 1 && ITEMS * 8 <= 32, "one key word; one warp scans the counts");
+    __shared__ unsigned s_w[8], s_cnt[ITEMS * 8], s_total;
+    __shared__ unsigned long long s_base;
+    __shared__ unsigned s_z[256 * ITEMS], s_o[256 * ITEMS];  // entry with target bit 0, with 1; ~0: none
+    const unsigned flags = *d.flags;
+    if (flags & kPairStray) {  // the host takes the hashed table
+        if (blockIdx.x == 0 && threadIdx.x == 0) *a.cursor = ~0ull;
+        return;
+    }
+    const bool split = (flags & 3u) == 3u;
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint64_t bit = 1ull << a.target.shift;
+    const uint64_t stride = (uint64_t)gridDim.x * (256u * ITEMS);
+    for (uint64_t b = (uint64_t)blockIdx.x * (256u * ITEMS); b < n; b += stride) {
+        unsigned copy = 0;
+        unsigned z[ITEMS], o[ITEMS];
+        {
+            uint64_t k[ITEMS][1];
+            unsigned own[ITEMS], mate[ITEMS];
+#pragma unroll
+            for (int q = 0; q < ITEMS; ++q) {
+                const uint64_t i = b + (uint64_t)q * 256u + threadIdx.x;
+                k[q][0] = i < n ? __ldg(a.in_keys.w[0] + i) : 0ull;
+            }
+#pragma unroll
+            for (int q = 0; q < ITEMS; ++q) {
+                const uint64_t i = b + (uint64_t)q * 256u + threadIdx.x;
+                own[q] = mate[q] = z[q] = o[q] = ~0u;
+                if (i >= n) continue;
+                if (!cond_ok<1>(k[q], cond)) {
+                    copy |= 1u << q;
+                    continue;
+                }
+                if (k[q][0] & bit) o[q] = (unsigned)i;
+                else z[q] = (unsigned)i;
+                if (!split) continue;
+                own[q] = d.slot[(k[q][0] >> d.lo) & d.mask];
+                mate[q] = d.slot[((k[q][0] ^ bit) >> d.lo) & d.mask];
+            }
+#pragma unroll
+            for (int q = 0; q < ITEMS; ++q) {
+                const uint64_t i = b + (uint64_t)q * 256u + threadIdx.x;
+                uint64_t p[1] = {k[q][0] ^ bit};
+                if ((z[q] & o[q]) == ~0u || own[q] != (unsigned)i || mate[q] >= n) continue;
+                if (__ldg(a.in_keys.w[0] + mate[q]) != p[0] || !cond_ok<1>(p, cond)) continue;
+                if (z[q] != ~0u) o[q] = mate[q];
+                else o[q] = ~0u;  // its partner's thread computes the pair
+            }
+        }
+        unsigned ball[ITEMS];
+#pragma unroll
+        for (int q = 0; q < ITEMS; ++q) {
+            ball[q] = __ballot_sync(0xffffffffu, (z[q] & o[q]) != ~0u);
+            if (lane == 0) s_cnt[q * 8 + warp] = __popc(ball[q]);
+        }
+        const int copies = __syncthreads_or(copy);
+        if (warp == 0) {
+            const unsigned c = lane < ITEMS * 8 ? s_cnt[lane] : 0u;
+            unsigned inc = c;
+#pragma unroll
+            for (int t = 1; t < 32; t <<= 1) {
+                const unsigned v = __shfl_up_sync(0xffffffffu, inc, t);
+                if (lane >= (unsigned)t) inc += v;
+            }
+            if (lane < ITEMS * 8) s_cnt[lane] = inc - c;
+            if (lane == 31u) s_total = inc;
+        }
+        __syncthreads();
+        const unsigned total = s_total;
+#pragma unroll
+        for (int q = 0; q < ITEMS; ++q) {
+            if (!((ball[q] >> lane) & 1u)) continue;
+            const unsigned at = s_cnt[q * 8 + warp] + __popc(ball[q] & ((1u << lane) - 1u));
+            s_z[at] = z[q];
+            s_o[at] = o[q];
+        }
+        __syncthreads();
+        if (copies) {
+            bool fits;
+            unsigned long long at = block_reserve<256>(a, __popc(copy), s_w, &s_base, fits);
+#pragma unroll
+            for (int q = 0; q < ITEMS; ++q) {
+                if (!fits || !((copy >> q) & 1u)) continue;
+                const uint64_t i = b + (uint64_t)q * 256u + threadIdx.x;
+                uint64_t k[1];
+                load_key<1>(a.in_keys, (unsigned)i, k);
+                store_out<1>(a, at++, k, a.in_amp[i]);
+            }
+        }
+        for (unsigned p0 = 0; p0 < total; p0 += 256u) {
+            const unsigned p = p0 + threadIdx.x;
+            uint64_t k[1];
+            double2 rz, ro;
+            bool kz = false, ko = false;
+            if (p < total) {
+                const unsigned iz = s_z[p], io = s_o[p];
+                const bool hz = iz != ~0u, ho = io != ~0u;
+                const double2 zero = make_double2(0.0, 0.0);
+                load_key<1>(a.in_keys, hz ? iz : io, k);
+                pair_math<1>(a, k, hz ? a.in_amp[iz] : zero, ho ? a.in_amp[io] : zero, hz, ho, rz, ro, kz, ko);
+            }
+            bool fits;
+            const unsigned long long at = block_reserve<256>(a, (unsigned)kz + (unsigned)ko, s_w, &s_base, fits);
+            if (fits && (kz || ko)) store_pair<1>(a, at, k, rz, ro, kz, ko);
+        }
+        __syncthreads();
+    }
+}
+
 // The whole split of a small state in one CTA: the table lives in shared
 // memory, members of a pair learn of each other there, and the outputs are
 // written in entry order with their number posted to the host by the same
@@ -3544,6 +3710,50 @@ static unsigned cond_words(const DCondSet& c) {
     return m;
 }
 
+// A table of the registers' bits pays while it stays in L2 (2^24 slots: 64 MB)
+// or has at most four slots per entry (the hashed table takes 12 to 24 bytes
+// per entry). A split of a dense 2^21-entry state: 65 us of kernels, 125
+// through the hashed table; of the QDA walk's 0.1 to 2 M entries over 24 bits:
+// 35 us on average against 66.
+constexpr unsigned kPairDirectBits = 24;
+
+// The split through PairDirect; false when the keys do not fit it or hold bits
+// of registers that are gone (T is set otherwise).
+template <int K>
+static bool pair_direct(uint64_t N, const GroupSpec& gs, EmitArgs& ea, unsigned long long* cur, unsigned long long& T) {
+    if constexpr (K != 1) {
+        return false;
+    } else {
+        uint64_t active[SQ_KMAX];
+        regtable().active_mask(active);
+        if (!active[0] || regtable().k != 1) return false;
+        PairDirect d;
+        d.lo = (unsigned)__builtin_ctzll(active[0]);
+        const unsigned bits = 64u - (unsigned)__builtin_clzll(active[0]) - d.lo;
+        if (bits > kPairDirectBits && (bits > 32u || (1ull << bits) > 4 * N)) return false;
+        d.mask = (1ull << bits) - 1ull;
+        d.slot = (unsigned*)ws().get(WS_PAIR_TABLE, 4ull << bits);
+        d.flags = (unsigned*)(cur + 1);
+        cudaStream_t st = stream();
+        SQ_CUDA(cudaMemsetAsync(cur, 0, 16, st));
+        prof_begin("pair_scatter");
+        pair_scatter_kernel<K><<<grid_for(N, 1024, 8), 256, 0, st>>>(ea.in_keys, N, gs.cond, gs.target, d);
+        prof_end((double)N * 12);
+        prof_begin("pair_direct");
+        // two entries per thread once that still fills the SMs; a CTA per tile up to 64 per SM
+        if (N >= (uint64_t)num_sms() * 512)
+            pair_direct_kernel<K, 2><<<grid_for((N + 1) / 2, 256, 64), 256, 0, st>>>(ea, N, gs.cond, d);
+        else
+            pair_direct_kernel<K, 1><<<grid_for(N, 256, 64), 256, 0, st>>>(ea, N, gs.cond, d);
+        prof_end((double)N * 24);
+        SQ_CUDA(cudaGetLastError());
+        host_read(&T, cur, 8);
+        if (T != ~0ull) return true;
+        T = 0;
+        return false;
+    }
+}
+
 // Pair split by partner lookup; outputs at most 2N (two per passing entry,
 // one per copied entry). Up to kPairSmallMax entries one CTA does everything:
 // from call to call (RY, one key word) 16 us against 34 through the table at
@@ -3574,7 +3784,7 @@ static void run_pair_partner(State& s, const GroupSpec& gs, EmitArgs& ea) {
         prof_end((double)N * (8.0 * K + 16));
         SQ_CUDA(cudaGetLastError());
         mail_read(mail, &T, cur, 8);
-    } else {
+    } else if (!pair_direct<K>(N, gs, ea, cur, T)) {
         PairTable t;
         const uint64_t met16 = (N + 15) / 16;
         t.slots = (unsigned long long*)ws().get(WS_PAIR_TABLE, cap * 8 + met16 * 16);
