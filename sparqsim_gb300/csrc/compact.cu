@@ -52,8 +52,9 @@ struct KeySelect {
 // Whether ClearZero has anything to drop. Every split prunes its outputs at the
 // same threshold, so the ClearZero calls that the walks make after them almost
 // never do: 16 bytes read per entry instead of 24 K + 48 (read, and written to
-// the other buffer). A CKS term's four calls at 2.6 M entries of six words:
-// 410 us of kernels in one pass, 60 when the check lets them be skipped.
+// the other buffer). A call at 2.6 M entries of six words: 160 us before, 26
+// when nothing goes; when something does, the check adds its 15 us to 124 of
+// compaction.
 __global__ void __launch_bounds__(kCzBlock) prune_any_kernel(const double2* __restrict__ a, uint64_t n, double eps,
                                                              unsigned* __restrict__ any) {
     const uint64_t stride = (uint64_t)gridDim.x * kCzTile;
@@ -467,7 +468,8 @@ void settle_swap(State& s) {
 // finishes last sums the CTAs' results in their order (norm_final's), so the
 // value does not depend on timing; it posts it to the host. Two fused
 // multiply-adds per entry: the FP64 pipe (2 lanes per SM and clock) was the
-// bound with two products and two sums (2.6 M entries: 20 us, 13 here).
+// bound with two products and two sums (2.6 M entries: two launches of 30 and
+// 6 us, event overhead included; 21 here; Normalize 66 -> 45 us per call).
 // ticket: zero between launches.
 __global__ void __launch_bounds__(kRedBlock) norm_kernel(const double2* __restrict__ a, uint64_t n,
                                                          double* __restrict__ partial, unsigned* ticket,

@@ -491,10 +491,11 @@ __device__ __forceinline__ void exec(const DInstr& in, R (&kk)[Q], double2 (&aa)
 // results are kept modulo 2^32 or less, so 32-bit arithmetic gives the same
 // bits, and a field costs one funnel shift and one AND. The first 8 bytes of a
 // field (word, shift, mask) are one constant load. A 9-operator chain over
-// 32-bit registers, 2^23 entries of two key words: 215 us in 64-bit arithmetic,
-// 165 here; both are bound by integer issue (the ALU pipe 69 to 75 % busy).
-// Keeping the fields in shared-memory slots while a program runs was measured
-// too (205 us).
+// 32-bit registers, 2^23 entries of two key words: 207 us per pass against 260
+// with 64-bit fields selected among all the state's words and one condition
+// test each; both are bound by integer issue (the ALU pipe 69 to 75 % busy).
+// Keeping the fields in shared-memory slots while a program runs was slower:
+// compute, phase and uncompute 603 us against 515.
 struct NField {
     unsigned word, shift;
     uint32_t mask;
@@ -692,7 +693,8 @@ static void launch_program(const ProgramArgs<MAXI>& args, const LocalKeys& keys,
 template <int K, int MAXI>
 static void dispatch_q(const ProgramArgs<MAXI>& args, const LocalKeys& keys, State& s, double tb) {
     // two entries per thread once that still gives every SM its warps (four
-    // were slower at two key words, 185 against 165 us for the chain above)
+    // were slower at two key words: compute, phase and uncompute of the chain
+    // above 564 us against 515)
     constexpr int Q = 2;
     if (s.n >= (uint64_t)num_sms() * 2048 * Q) launch_program<K, Q, MAXI>(args, keys, s, tb);
     else launch_program<K, 1, MAXI>(args, keys, s, tb);

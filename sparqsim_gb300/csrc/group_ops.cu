@@ -3212,8 +3212,8 @@ static Grouping group_by_hash(State& s, const GroupSpec& gs, uint64_t* dg, uint6
 // table no longer fits L2, 555 and 231 us) and the output reservations (0.7 ns
 // per atomic on one address). A build pass followed by a lookup pass costs two
 // random accesses and one key comparison per entry more: 179 us of kernels per
-// split of a dense 2^21-entry state against 125 us (flags 6, clear 6, claim 95,
-// lone 4, event overheads included) in this form.
+// split of a dense 2^21-entry state against 125 us (flags 10, clear 10, claim 97,
+// lone 8, event overheads included) in this form.
 struct PairTable {
     unsigned long long* slots;
     unsigned long long mask;  // capacity - 1
