@@ -2360,7 +2360,7 @@ __device__ __forceinline__ unsigned block_rank(unsigned c, unsigned* s, unsigned
 struct HashWs {
     unsigned long long* slots;
     unsigned long long cap_mask;
-    unsigned* gcount;     // [0]: groups, [1]: entries failing the conditions, [2]: table overflow
+    unsigned* gcount;     // [0]: groups, [1]: entries failing the conditions, [2]: table overflow, [3]: sampled claims
     unsigned* cnt;        // per slot: members besides the head; after the scan: the group's next free position
     unsigned* head;       // one entry per group
     unsigned* gid;        // slot of each entry (~0u: fails the conditions)
@@ -2383,10 +2383,15 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
 
 // gmax: groups that the table may hold (half of its slots). More raise the
 // overflow flag, which ends the launch's remaining work; the host retries.
+// A CTA counts its claims at the end of its round, which it does not reach
+// while one of its lanes probes a full table: claims of every 64th slot are
+// counted as they are made, and past `early` of them (times 64; three quarters
+// of the slots, ~0 when every entry fits) the flag is raised at once. A split
+// of 400,000 groups whose number was predicted too low took 4 to 11 ms without this.
 template <int K>
 __global__ void __launch_bounds__(256) hash_insert_kernel(ConstKeyPtrs keys, const uint64_t* __restrict__ gmask,
                                                           DCondSet cond, uint64_t n, HashWs h, unsigned gmax,
-                                                          Field tgt, Field varw, unsigned max_digits, unsigned* err) {
+                                                          unsigned early, Field tgt, Field varw, unsigned max_digits, unsigned* err) {
     __shared__ unsigned s_fail[8];
     __shared__ unsigned s_fail_base;
     uint64_t gm[K];
@@ -2450,6 +2455,8 @@ __global__ void __launch_bounds__(256) hash_insert_kernel(ConstKeyPtrs keys, con
                 const unsigned long long v = atomicCAS(&h.slots[slot], 0ull, tag);
                 claimed = v == 0ull;
                 bool eq = claimed;
+                if (claimed && early != ~0u && (slot & 63ull) == 0ull && atomicAdd(&h.gcount[3], 64u) + 64u > early)
+                    h.gcount[2] = 1u;
                 if (!claimed && (v >> 32) == (tag >> 32)) {
                     const unsigned hidx = (unsigned)(v & 0xffffffffull) - 1u;
                     uint64_t hk[K];
@@ -3160,8 +3167,9 @@ static Grouping group_by_hash(State& s, const GroupSpec& gs, uint64_t* dg, uint6
         unsigned* seg = (unsigned*)ws().get(WS_SEG, (most + 2) * 4);
         SQ_CUDA(cudaMemsetAsync(base, 0, off_head, st));  // slots, counters, cnt
         prof_begin("hash_insert");
-        hash_insert_kernel<K><<<grid_for(N, 256, 8), 256, 0, st>>>(ik, dg, gs.cond, N, h, (unsigned)(cap / 2), gs.target,
-                                                                   gs.varw, gs.target.width, device_error_word());
+        hash_insert_kernel<K><<<grid_for(N, 256, 8), 256, 0, st>>>(
+            ik, dg, gs.cond, N, h, (unsigned)(cap / 2), want < N ? (unsigned)(cap / 4 * 3) : ~0u, gs.target, gs.varw,
+            gs.target.width, device_error_word());
         prof_end((double)N * (8.0 * K + 4));
         SQ_CUDA(cudaGetLastError());
         const long long nt = (long long)((cap + kSelTile - 1) / kSelTile);
