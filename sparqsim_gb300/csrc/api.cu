@@ -340,8 +340,9 @@ int sq_state_copy(sq_state* dst, const sq_state* src) {
     }
     SQ_CUDA(cudaMemcpyAsync(d.live.amp, s.live.amp, s.n * 16, cudaMemcpyDeviceToDevice, stream()));
     d.n = s.n;
-    std::copy(s.zeroed, s.zeroed + SQ_KMAX, d.zeroed);
-    for (uint32_t w = k; w < SQ_KMAX; ++w) d.zeroed[w] = 0;  // words that were not copied
+    uint64_t active[SQ_KMAX];
+    regtable().active_mask(active);
+    for (uint32_t w = 0; w < SQ_KMAX; ++w) d.zeroed[w] = w < k ? s.zeroed[w] & ~active[w] : 0;  // words past k were not copied
     SQ_API_END
 }
 
@@ -1554,6 +1555,7 @@ int sq_remove_register_sync(sq_state* st, uint32_t id) {
     Field f = regtable().field(id);
     zero_field(s, f);
     regtable().remove(id);
+    if (f.width) s.zeroed[f.word] |= wmask(f.width) << f.shift;  // inactive from here on: nothing writes them
     SQ_API_END
 }
 

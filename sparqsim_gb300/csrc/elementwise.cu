@@ -1120,7 +1120,6 @@ void zero_field(State& s, Field f) {
     if (s.n == 0 || f.width == 0) return;
     const uint64_t keep = ~(wmask(f.width) << f.shift);
     if (!(~keep & ~s.zeroed[f.word])) return;  // cleared when its last register was removed
-    s.zeroed[f.word] |= ~keep;
     prof_begin("zero_field");
     zero_field_kernel<1><<<grid_for(s.n, 256), 256, 0, stream()>>>(s.live.keys[f.word], keep, s.n);
     prof_end((double)s.n * 16);
@@ -1149,6 +1148,7 @@ __global__ void move_field_kernel(KeyPtrs keys, Field first, Field second, Field
 void move_field(State& s, Field first, Field second, Field dst) {
     drop_groups(s);
     sync_words(s);
+    s.zeroed[dst.word] &= ~(wmask(dst.width) << dst.shift);  // may lie over bits cleared by an earlier removal
     if (s.n == 0) return;
     KeyPtrs kp;
     for (int w = 0; w < SQ_KMAX; ++w) kp.w[w] = s.live.keys[w];

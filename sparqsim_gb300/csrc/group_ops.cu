@@ -4631,7 +4631,9 @@ void add_systems(State& dst, const State& src, double coef) {
     if (src.n == 0) return;
     sync_words(dst);
     const uint32_t k = regtable().k;
-    for (int w = 0; w < SQ_KMAX; ++w) dst.zeroed[w] &= src.zeroed[w];
+    uint64_t active[SQ_KMAX];
+    regtable().active_mask(active);
+    for (int w = 0; w < SQ_KMAX; ++w) dst.zeroed[w] &= src.zeroed[w] & ~active[w];
     const uint64_t n0 = dst.n, n1 = src.n;
     const int do_scale = std::abs(coef - 1.0) > 1e-14 ? 1 : 0;
     // the join, unless the size model is logging merges too (the grouped path does)

@@ -213,10 +213,14 @@ struct State {
     Buffers live;
     Buffers spare;
     uint64_t n = 0;
-    // Bits of inactive registers known to be 0 in every entry: what zero_field
-    // has cleared and no register covers since. A register that gets such bits
-    // needs no clearing pass (drivers remove and add the same scratch registers
-    // tens of times per walk step).
+    // Bits of inactive registers known to be 0 in every entry: those of a
+    // register that was removed together with this state, until a register
+    // covers them again. A register that gets such bits needs no clearing pass
+    // (drivers remove and add the same scratch registers tens of times per walk
+    // step). Only the removal sets them: the calls that make a register may
+    // write it before they return. Every entry point drops those that an active
+    // register covers (S() in api.cu); one that makes bits active and writes
+    // them itself drops them there (move_field).
     uint64_t zeroed[SQ_KMAX] = {0};
     GroupCache groups;
     // A ClearZero that drops nothing leaves the entries where they are instead
