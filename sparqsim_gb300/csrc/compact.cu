@@ -23,9 +23,10 @@ struct LookbackWs {
     unsigned long long* status;
     unsigned* counter;
     unsigned long long* total;
+    unsigned* done;  // tiles whose survivors are stored
 };
 
-// Layout of the look-back workspace: [counter (u32) | total (u64) | pad to 256 B | status[ntiles]].
+// Layout of the look-back workspace: [counter (u32) | total (u64) | any (u32) | done (u32) | pad to 256 B | status[ntiles]].
 // One tile waits for none and takes no ticket: its words need no clearing.
 static LookbackWs lookback_ws(long long ntiles) {
     size_t bytes = 256 + (size_t)ntiles * 8;
@@ -34,6 +35,7 @@ static LookbackWs lookback_ws(long long ntiles) {
     LookbackWs w;
     w.counter = (unsigned*)p;
     w.total = (unsigned long long*)(p + 8);
+    w.done = (unsigned*)(p + 20);
     w.status = (unsigned long long*)(p + 256);
     return w;
 }
@@ -77,7 +79,8 @@ constexpr unsigned long long kCzUnchanged = 1ull << 63;
 // SEL = false: ClearZero (keep |a|^2 >= eps); SEL = true: keep the entries the
 // key selection accepts. Same single pass either way. any: prune_any's word
 // (null: compact whatever it would say); the number of survivors, or n |
-// kCzUnchanged when nothing was written, is posted to the host.
+// kCzUnchanged when nothing was written, is posted to the host, by the CTA that
+// finishes last: the host returns to a caller who may read the entries.
 template <int K, bool SEL>
 __global__ void __launch_bounds__(kCzBlock) clearzero_kernel(ConstKeyPtrs ik, const double2* __restrict__ ia,
                                                              KeyPtrs ok, double2* __restrict__ oa, uint64_t n,
@@ -139,10 +142,7 @@ __global__ void __launch_bounds__(kCzBlock) clearzero_kernel(ConstKeyPtrs ik, co
         unsigned long long pre = lb_warp_exclusive(lb.status, tile, total, err);
         if (lane == 0) {
             s_prefix = pre;
-            if (tile == ntiles - 1) {
-                *lb.total = pre + total;
-                mail_post(mail, pre + total);
-            }
+            if (tile == ntiles - 1) *lb.total = pre + total;
         }
     }
     __syncthreads();
@@ -156,6 +156,15 @@ __global__ void __launch_bounds__(kCzBlock) clearzero_kernel(ConstKeyPtrs ik, co
 #pragma unroll
         for (int w = 0; w < K; ++w) ok.w[w][o] = ik.w[w][i];
         oa[o] = a[j];
+    }
+    if (!mail.mail) return;
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        if (ntiles == 1 || atomicAdd(lb.done, 1u) == (unsigned)ntiles - 1u) {
+            __threadfence();
+            mail_post(mail, *reinterpret_cast<volatile unsigned long long*>(lb.total));
+        }
     }
 }
 
@@ -599,6 +608,7 @@ static void launch_cz_noalloc(const uint64_t* const* keys_in, const double* amps
     LookbackWs lb;
     lb.counter = (unsigned*)scratch;
     lb.total = scratch + 1;
+    lb.done = nullptr;  // nothing is posted
     lb.status = scratch + kNoAllocHeaderWords;
     KeySelect none;
     memset(&none, 0, sizeof(none));

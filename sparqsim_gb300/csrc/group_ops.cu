@@ -3701,6 +3701,7 @@ __global__ void __launch_bounds__(BLOCK) pair_small_kernel(const __grid_constant
         if (copy) store_out<K>(a, o, k, rz);
         else if (kz || ko) store_pair<K>(a, o, k, rz, ro, kz, ko);
     }
+    __syncthreads();  // every output is stored: the host returns to a caller who may read them
     if (tid == 0) {
         *a.cursor = base;
         mail_post(mail, base);

@@ -314,7 +314,10 @@ __device__ __forceinline__ void mail_seal(unsigned char* mail, const unsigned* e
     __threadfence_system();
     *reinterpret_cast<volatile unsigned long long*>(mail) = seq;
 }
-// One thread, after every store and error flag of the operator is visible to it.
+// One thread, after a barrier (or a counter of finished CTAs, with fences)
+// behind every error flag of the kernel and every store to the state: the host
+// takes the letter for the end of the operator and returns. Stores to the
+// workspace, which only later launches read, may still be under way.
 __device__ __forceinline__ void mail_post(const MailSlot& m, unsigned long long v) {
     if (!m.mail) return;
     *reinterpret_cast<volatile unsigned long long*>(m.mail + kMailData) = v;
