@@ -829,18 +829,23 @@ void ensure_buffers(Buffers& b, uint64_t cap, uint32_t k, uint64_t keep) {
     b = nb;
 }
 
-__global__ void ground_state_kernel(KeyPtrs keys, unsigned words, double2* amp) {
+__global__ void ground_state_kernel(KeyPtrs keys, unsigned words, double2* amp, const __grid_constant__ MailSlot mail) {
     if (threadIdx.x < words) keys.w[threadIdx.x][0] = 0ull;
     if (threadIdx.x == 0) *amp = make_double2(1.0, 0.0);
+    __syncthreads();
+    if (threadIdx.x == 0) mail_post(mail, 1ull);
 }
 
 void ground_state(State& s) {
     KeyPtrs kp;
     for (int w = 0; w < SQ_KMAX; ++w) kp.w[w] = s.live.keys[w];
-    ground_state_kernel<<<1, SQ_KMAX, 0, stream()>>>(kp, s.live.kalloc, s.live.amp);
+    const MailSlot mail = mail_slot();
+    ground_state_kernel<<<1, SQ_KMAX, 0, stream()>>>(kp, s.live.kalloc, s.live.amp, mail);
     SQ_CUDA(cudaGetLastError());
     count_launch();
-    s.n = 1;
+    unsigned long long n = 0;
+    mail_read(mail, &n, nullptr, sizeof(n));  // callers never run under capture
+    s.n = n;
 }
 
 void sync_words(State& s) {

@@ -358,7 +358,7 @@ void ensure_buffers(Buffers& b, uint64_t cap, uint32_t k, uint64_t keep);
 // Make the state's live buffers hold K = regtable().k words.
 void sync_words(State& s);
 void free_buffers(Buffers& b);
-// The single entry |0...0>, amplitude 1, in the live buffers (one launch; nothing waits for it).
+// The single entry |0...0>, amplitude 1, in the live buffers, written on return.
 void ground_state(State& s);
 void swap_live_spare(State& s);
 

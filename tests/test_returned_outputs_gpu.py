@@ -80,3 +80,20 @@ def test_splits(other, n, words):
     for step in range(12):
         ps.RY_Bool("q", step % 3, 0.3 + 0.1 * step)(st)
         _same(st, other)
+
+
+@pytest.mark.parametrize("words", [1, 8])
+def test_new_and_reset_states(other, words):
+    for w in range(words):
+        ps.System.add_register(f"p{w}", U, 64)
+    st = ps.SparseState()
+    for step in range(20):
+        fresh = ps.SparseState()
+        keys_amp = _read(fresh, other)
+        assert all(int(k[0]) == 0 for k in keys_amp[:-1]) and complex(keys_amp[-1][0]) == 1
+        for w in range(words):
+            ps.Init_Unsafe(f"p{w}", step + 1)(st)
+        ps.GlobalPhase(1j)(st)
+        st.reset()
+        keys_amp = _read(st, other)
+        assert all(int(k[0]) == 0 for k in keys_amp[:-1]) and complex(keys_amp[-1][0]) == 1
