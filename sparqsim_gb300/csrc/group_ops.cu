@@ -3207,7 +3207,7 @@ static Grouping group_by_hash(State& s, const GroupSpec& gs, uint64_t* dg, uint6
 
 // ------------------------------------------------------------------ pair splits by partner lookup
 // A 1-bit split pairs each entry with the entry whose key differs in the
-// target bit alone (keys are unique). No grouping: members of a pair meet in
+// target bit alone. No grouping: members of a pair meet in
 // an open-addressing table on the key without the target bit. The first to
 // arrive leaves its index in the slot; the second finds it there, knows both
 // members and writes the pair's outputs at once (pair_math, the arithmetic of
@@ -3227,6 +3227,7 @@ struct PairTable {
     unsigned long long mask;  // capacity - 1
     unsigned* flags;          // bit 0: a passing entry has target bit 0, bit 1: one has 1
     unsigned char* met;       // 1: the entry found its partner
+    unsigned long long* seen; // entries accounted for: two per pair, one per copied or lone entry
 };
 template <int K>
 __device__ __forceinline__ unsigned long long full_key_hash(const uint64_t (&k)[K]) {
@@ -3250,6 +3251,25 @@ __device__ __forceinline__ bool is_partner(const ConstKeyPtrs& keys, unsigned lo
 #pragma unroll
     for (int w = 0; w < K; ++w) eq = eq && __ldg(keys.w[w] + j) == ((unsigned)w == tw ? k[w] ^ bit : k[w]);
     return eq;
+}
+
+// Marks entry j as met. TAKE: false if another entry met it before.
+template <bool TAKE>
+__device__ __forceinline__ bool meet(const PairTable& t, unsigned j) {
+    if (!TAKE) {
+        t.met[j] = 1;
+        return true;
+    }
+    const unsigned m = 1u << (8u * (j & 3u));
+    return !(atomicOr(reinterpret_cast<unsigned*>(t.met) + (j >> 2), m) & m);
+}
+
+// Adds a CTA's count of entries to *total. s: one word per warp.
+template <int BLOCK>
+__device__ __forceinline__ void block_tally(unsigned c, unsigned* s, unsigned long long* total) {
+    unsigned sum;
+    (void)block_rank<BLOCK>(c, s, sum);
+    if (threadIdx.x == 0 && sum) atomicAdd(total, (unsigned long long)sum);
 }
 
 // One reservation on the output cursor per CTA (a reservation per warp put
@@ -3328,7 +3348,15 @@ static __global__ void __launch_bounds__(256) pair_clear_kernel(PairTable t, uin
 // lane active as for a full one. Failing entries are copied. ITEMS entries
 // per thread keep their table accesses in flight together and share one
 // output reservation.
-template <int K, int ITEMS>
+//
+// A state may hold a key several times (uploaded so, or after a register was
+// removed that told its entries apart). Two copies that meet the same partner
+// would both count it; then `seen` is more than the entries there are, and the
+// host runs the split again with TAKE, where a partner is taken by one entry and
+// passed over by the others, which stay lone. Taking always costs an atomic
+// with a result per pair: 158 us per split of 2^20 entries of two key words
+// against 145.
+template <int K, int ITEMS, bool TAKE = false>
 __global__ void __launch_bounds__(256) pair_claim_kernel(const __grid_constant__ EmitArgs a, uint64_t n,
                                                          const __grid_constant__ DCondSet cond, PairTable t) {
     __shared__ unsigned s_w[8];
@@ -3337,6 +3365,7 @@ __global__ void __launch_bounds__(256) pair_claim_kernel(const __grid_constant__
     if ((*t.flags & 3u) != 3u) return;
     const unsigned tw = a.target.word;
     const uint64_t bit = 1ull << a.target.shift;
+    unsigned seen = 0;
     const uint64_t stride = (uint64_t)gridDim.x * (256u * ITEMS);
     for (uint64_t b = (uint64_t)blockIdx.x * (256u * ITEMS); b < n; b += stride) {
         unsigned copy = 0, found = 0;  // bit q: item q fails the conditions / met its partner
@@ -3371,18 +3400,19 @@ __global__ void __launch_bounds__(256) pair_claim_kernel(const __grid_constant__
                 // at most capacity probes; the table is never full
                 for (unsigned long long probes = 0; v[q] != 0ull && probes <= t.mask; ++probes) {
                     if ((v[q] >> 32) == (tag[q] >> 32) &&
-                        is_partner<K>(a.in_keys, (v[q] & 0xffffffffull) - 1ull, k[q], tw, bit)) {
+                        is_partner<K>(a.in_keys, (v[q] & 0xffffffffull) - 1ull, k[q], tw, bit) &&
+                        meet<TAKE>(t, (unsigned)(v[q] & 0xffffffffull) - 1u)) {
                         partner[q] = (unsigned)(v[q] & 0xffffffffull) - 1u;
                         found |= 1u << q;
                         if (kword<K>(k[q], tw) & bit) one |= 1u << q;
                         t.met[b + (uint64_t)q * 256u + threadIdx.x] = 1;
-                        t.met[partner[q]] = 1;
                         break;
                     }
                     slot[q] = (slot[q] + 1) & t.mask;
                     v[q] = atomicCAS(&t.slots[slot[q]], 0ull, tag[q]);
                 }
             }
+            seen += __popc(copy) + 2u * __popc(found);
         }
         unsigned pairs;
         unsigned at = block_rank<256>(__popc(found), s_w, pairs);
@@ -3423,6 +3453,7 @@ __global__ void __launch_bounds__(256) pair_claim_kernel(const __grid_constant__
         }
         __syncthreads();
     }
+    block_tally<256>(seen, s_w, t.seen);
 }
 
 // The entries not written by the claim pass: the passing entries that met no
@@ -3436,6 +3467,7 @@ __global__ void __launch_bounds__(256) pair_lone_kernel(const __grid_constant__ 
     const bool claimed = (*t.flags & 3u) == 3u;
     const unsigned tw = a.target.word;
     const uint64_t bit = 1ull << a.target.shift;
+    unsigned seen = 0;
     const uint64_t stride = (uint64_t)gridDim.x * 1024u;
     for (uint64_t b0 = (uint64_t)blockIdx.x * 1024u; b0 < n; b0 += stride) {
         unsigned mine = 0;  // bit q: entry b0 + 256 q + thread is left
@@ -3444,6 +3476,7 @@ __global__ void __launch_bounds__(256) pair_lone_kernel(const __grid_constant__ 
             const uint64_t i = b0 + (uint64_t)q * 256u + threadIdx.x;
             if (i < n && !(claimed && t.met[i])) mine |= 1u << q;
         }
+        seen += __popc(mine);
         if (!__syncthreads_or(mine)) continue;
         for (int q = 0; q < 4; ++q) {
             const uint64_t i = b0 + (uint64_t)q * 256u + threadIdx.x;
@@ -3469,6 +3502,7 @@ __global__ void __launch_bounds__(256) pair_lone_kernel(const __grid_constant__ 
             else if (kz || ko) store_pair<K>(a, o, k, rz, ro, kz, ko);
         }
     }
+    block_tally<256>(seen, s_w, t.seen);
 }
 
 // Where the registers span few enough bits of a one-word key, the bits
@@ -3668,9 +3702,9 @@ __global__ void __launch_bounds__(BLOCK) pair_small_kernel(const __grid_constant
         for (unsigned probes = 0; probes < cap; ++probes) {  // never full: ends at an empty slot
             const unsigned old = atomicCAS(&table[slot], 0u, e + 1u);
             if (old == 0u) break;
-            if (is_partner<K>(a.in_keys, old - 1u, k, tw, bit)) {
+            // a partner that another copy of this key has met is passed over
+            if (is_partner<K>(a.in_keys, old - 1u, k, tw, bit) && atomicCAS(&mate[old - 1u], 0u, e + 1u) == 0u) {
                 mate[e] = old;
-                mate[old - 1u] = e + 1u;
                 break;
             }
             slot = (slot + 1u) & (cap - 1u);
@@ -3799,9 +3833,10 @@ static void run_pair_partner(State& s, const GroupSpec& gs, EmitArgs& ea) {
         t.slots = (unsigned long long*)ws().get(WS_PAIR_TABLE, cap * 8 + met16 * 16);
         t.mask = cap - 1;
         t.met = (unsigned char*)(t.slots + cap);
-        t.flags = (unsigned*)(cur + 1);
+        t.seen = cur + 1;
+        t.flags = (unsigned*)(cur + 2);
         if (N > kPairFlagsMin) {
-            SQ_CUDA(cudaMemsetAsync(cur, 0, 16, st));
+            SQ_CUDA(cudaMemsetAsync(cur, 0, 24, st));
             prof_begin("pair_flags");
             pair_flags_kernel<K><<<grid_for(N, 1024, 4), 256, 0, st>>>(ea.in_keys, N, dc, cond_words(dc) | (1u << gs.target.word),
                                                                        gs.target, t.flags);
@@ -3810,23 +3845,31 @@ static void run_pair_partner(State& s, const GroupSpec& gs, EmitArgs& ea) {
             pair_clear_kernel<<<grid_for(cap / 2, 256, 8), 256, 0, st>>>(t, met16);
             prof_end();
         } else {
-            SQ_CUDA(cudaMemsetAsync(cur, 0, 8, st));
+            SQ_CUDA(cudaMemsetAsync(cur, 0, 16, st));
             SQ_CUDA(cudaMemsetAsync(t.flags, 0xff, 4, st));
             SQ_CUDA(cudaMemsetAsync(t.slots, 0, cap * 8 + met16 * 16, st));
         }
-        prof_begin("pair_claim");
         // several entries per thread once that still fills the SMs
         constexpr int ITEMS = K <= 2 ? 4 : K <= 4 ? 2 : 1;
-        if (N >= (uint64_t)num_sms() * 256 * ITEMS)
-            pair_claim_kernel<K, ITEMS><<<grid_for((N + ITEMS - 1) / ITEMS, 256, 8), 256, 0, st>>>(ea, N, dc, t);
-        else
-            pair_claim_kernel<K, 1><<<grid_for(N, 256, 8), 256, 0, st>>>(ea, N, dc, t);
-        prof_end((double)N * (8.0 * K + 16));
-        prof_begin("pair_lone");
-        pair_lone_kernel<K><<<grid_for(N, 1024, 8), 256, 0, st>>>(ea, N, dc, t);
-        prof_end();
-        SQ_CUDA(cudaGetLastError());
-        host_read(&T, cur, 8);
+        const bool several = N >= (uint64_t)num_sms() * 256 * ITEMS;
+        for (bool take = false;; take = true) {
+            prof_begin("pair_claim");
+            if (take) pair_claim_kernel<K, 1, true><<<grid_for(N, 256, 8), 256, 0, st>>>(ea, N, dc, t);
+            else if (several) pair_claim_kernel<K, ITEMS><<<grid_for((N + ITEMS - 1) / ITEMS, 256, 8), 256, 0, st>>>(ea, N, dc, t);
+            else pair_claim_kernel<K, 1><<<grid_for(N, 256, 8), 256, 0, st>>>(ea, N, dc, t);
+            prof_end((double)N * (8.0 * K + 16));
+            prof_begin("pair_lone");
+            pair_lone_kernel<K><<<grid_for(N, 1024, 8), 256, 0, st>>>(ea, N, dc, t);
+            prof_end();
+            SQ_CUDA(cudaGetLastError());
+            unsigned long long r[2] = {0, 0};
+            host_read(r, cur, 16);
+            T = r[0];
+            if (r[1] == N || take) break;
+            // a partner was met twice: again, each taken once
+            SQ_CUDA(cudaMemsetAsync(cur, 0, 16, st));
+            SQ_CUDA(cudaMemsetAsync(t.slots, 0, cap * 8 + met16 * 16, st));
+        }
     }
     if (T > capT) fail(SQ_ERR_CAPACITY, "pair split wrote past its bound");
     prof_add_bytes_last((double)T * (8 * K + 16));
