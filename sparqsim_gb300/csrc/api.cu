@@ -318,6 +318,7 @@ int sq_state_reset(sq_state* st) {
     SQ_API_BEGIN
     State& s = S(st);
     drop_groups(s);
+    s.stray = 0;
     sync_words(s);
     ensure_buffers(s.live, 1, regtable().k, 0);
     if (capturing()) fail(SQ_ERR_CUDA, "capture: a state would be reset");
@@ -340,6 +341,7 @@ int sq_state_copy(sq_state* dst, const sq_state* src) {
     }
     SQ_CUDA(cudaMemcpyAsync(d.live.amp, s.live.amp, s.n * 16, cudaMemcpyDeviceToDevice, stream()));
     d.n = s.n;
+    d.stray = s.stray;
     uint64_t active[SQ_KMAX];
     regtable().active_mask(active);
     for (uint32_t w = 0; w < SQ_KMAX; ++w) d.zeroed[w] = w < k ? s.zeroed[w] & ~active[w] : 0;  // words past k were not copied
@@ -351,6 +353,7 @@ int sq_state_upload(sq_state* st, uint64_t n, const uint64_t* regs, uint32_t nre
     SQ_API_BEGIN
     State& s = S(st);
     drop_groups(s);
+    s.stray = 0;
     need(n == 0 || (regs != nullptr || nregs == 0) , "null regs");
     need(n == 0 || amps != nullptr, "null amps");
     const RegTable& t = regtable();
@@ -405,6 +408,7 @@ int sq_state_upload_packed(sq_state* st, uint64_t n, const uint64_t* keys, const
     SQ_API_BEGIN
     State& s = S(st);
     drop_groups(s);
+    s.stray = 0;
     need(n == 0 || (keys != nullptr && amps != nullptr), "null pointer");
     const uint32_t k = regtable().k;
     ensure_buffers(s.live, std::max<uint64_t>(n, 1), k, 0);
@@ -693,6 +697,7 @@ int sq_state_device_arrays(sq_state* st, uint64_t** key_words, uint32_t* k, doub
     State& s = S(st);
     drop_groups(s);  // the caller may write the arrays
     memset(s.zeroed, 0, sizeof(s.zeroed));
+    s.stray = 0;
     sync_words(s);
     if (key_words)
         for (uint32_t w = 0; w < regtable().k; ++w) key_words[w] = s.live.keys[w];

@@ -295,6 +295,7 @@ uint64_t compact_nonzero(const Buffers& in, Buffers& out, uint64_t n, double eps
 // their total probability. Returns that factor, or +inf when nothing is left.
 double select_entries(State& s, const DCondSet& sel, Field rf, uint64_t lo, uint64_t hi) {
     drop_groups(s);
+    s.stray = 0;  // the entries with such bits may be gone
     sync_words(s);
     if (s.n == 0) return 0.0;
     const uint32_t k = regtable().k;

@@ -1120,6 +1120,7 @@ void zero_field(State& s, Field f) {
     if (s.n == 0 || f.width == 0) return;
     const uint64_t keep = ~(wmask(f.width) << f.shift);
     if (!(~keep & ~s.zeroed[f.word])) return;  // cleared when its last register was removed
+    if (~keep & ~s.stray) s.stray = 0;  // bits outside the noted span are cleared
     prof_begin("zero_field");
     zero_field_kernel<1><<<grid_for(s.n, 256), 256, 0, stream()>>>(s.live.keys[f.word], keep, s.n);
     prof_end((double)s.n * 16);

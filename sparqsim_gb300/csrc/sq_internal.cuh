@@ -222,6 +222,11 @@ struct State {
     // register covers (S() in api.cu); one that makes bits active and writes
     // them itself drops them there (move_field).
     uint64_t zeroed[SQ_KMAX] = {0};
+    // The span of register bits (one key word) outside of which a 1-bit split has
+    // found set bits, of registers that are gone: the next split goes straight
+    // to the hashed table. 0: none found since the entries last came from
+    // elsewhere (upload, reset, a copy, the caller's writes) or bits were cleared.
+    uint64_t stray = 0;
     GroupCache groups;
     // A ClearZero that drops nothing leaves the entries where they are instead
     // of exchanging the buffers. Graphs are bound to the buffers' roles, which
