@@ -86,14 +86,14 @@ class System:
     # again when the engine's change counter has moved: operators look several
     # registers up by name each, and a call into the library per lookup was a
     # third of a small walk step's time.
-    _rows: list = []
+    _rows = None  # ctypes array, filled in place
+    _count = c_uint32()
     _by_name: dict = {}  # names looked up since the last change
     _seen = 0
     _changes = None
-    _buf = None
 
     @staticmethod
-    def _table() -> list:
+    def _table():
         c = System._changes
         if c is None or c.value != System._seen:
             System._refresh()
@@ -101,26 +101,28 @@ class System:
 
     @staticmethod
     def _refresh() -> None:
-        if System._buf is None:
-            System._buf = (c_uint32 * (5 * SQ_MAX_REGISTERS))()
-        n, p = c_uint32(), ctypes.POINTER(c_uint64)()
-        call("sq_system_snapshot", System._buf, len(System._buf) // 5, byref(n), byref(p))
-        System._changes = p.contents
-        System._rows, System._seen = System._buf[:5 * n.value], p.contents.value
+        if System._rows is None:
+            System._rows = (c_uint32 * (5 * SQ_MAX_REGISTERS))()
+            p = ctypes.POINTER(c_uint64)()
+            call("sq_system_snapshot", None, 0, byref(System._count), byref(p))
+            System._changes = p.contents
+        call("sq_system_snapshot", System._rows, SQ_MAX_REGISTERS, byref(System._count), None)
+        System._seen = System._changes.value
         System._by_name.clear()
 
     @staticmethod
     def _info(rid: int):
         rid = int(rid)
         rows = System._table()
-        if not 0 <= 5 * rid < len(rows):
+        if not 0 <= rid < System._count.value:
             call("sq_system_register_info", rid, None, None, None, None, None)  # raises: register not found
         t, w, a, wd, sh = rows[5 * rid:5 * rid + 5]
         return t, w, bool(a), wd, sh
 
     @staticmethod
     def register_count() -> int:
-        return len(System._table()) // 5
+        System._table()
+        return System._count.value
 
     @staticmethod
     def get_id(name: str) -> int:
@@ -128,7 +130,7 @@ class System:
         rid = System._by_name.get(name)
         if rid is not None:
             return rid
-        for rid in range(min(len(names), len(rows) // 5) - 1, -1, -1):
+        for rid in range(min(len(names), System._count.value) - 1, -1, -1):
             if names[rid] == name and rows[5 * rid + 2]:
                 System._by_name[name] = rid
                 return rid
