@@ -9,8 +9,11 @@
  *
  * Every entry point returns an sq_status (0 = success). No C++ exception crosses
  * this boundary; sq_last_error() returns a message for the last failure on the
- * calling thread. All calls are stream-ordered on the library's stream and are
- * synchronous with respect to the host where they return sizes.
+ * calling thread. All calls are stream-ordered on the library's stream; a call
+ * that returns or changes a size has the new size on the host when it returns.
+ * Its entries, like those of elementwise operators, may still be being written
+ * on that stream: a reader of sq_state_device_arrays on another stream first
+ * waits for sq_get_stream's, or calls sq_synchronize.
  *
  * Each declaration cites the reference interface it replaces (paths are relative
  * to the SparQSim project root). Register ids, condition kinds, XOR-out
@@ -209,8 +212,7 @@ int sq_init(int device);
 int sq_synchronize(void);
 /* The number of polls after which every bounded device-side wait gives up
  * (decoupled look-backs of ClearZero, group starts, count scans and the radix
- * sort's per-digit look-back; the hash grouping's wait on a locked slot): the
- * waiting block raises the device error word, finishes without waiting
+ * sort's per-digit look-back): the waiting block raises the device error word, finishes without waiting
  * further, and the next synchronising call returns SQ_ERR_DEVICE_TIMEOUT.
  * 0 restores the default, 2^22 polls. Stream-ordered: launches already
  * queued keep the limit they were queued with. No counterpart in the
@@ -485,10 +487,12 @@ int sq_hadamard_partial(sq_state* st, uint32_t reg, const uint32_t* positions, u
 /* ------------------------------------------------------------------ */
 /* Prune / norm / merge / register surgery                              */
 /* ------------------------------------------------------------------ */
-/* How split/merge operators group entries: 0 = automatic (hash grouping for
- * transforms on >= 4096 entries, sort otherwise; the add_systems merge always
- * sorts), 1 = onesweep radix sort, 2 = hash table. Results are identical;
- * only the entry order of the output differs. No counterpart in the reference
+/* How split/merge operators group entries: 0 = automatic (hash grouping; one
+ * CTA for small states), 1 = onesweep radix sort, 2 = hash table. Results are
+ * identical; only the entry order of the output differs. add_systems joins the
+ * two states by a hash table and sorts only when a state holds a key twice.
+ * 1-bit splits look partners up without a grouping under 0 and 3 (the default).
+ * No counterpart in the reference
  * (its CPU path sorts or uses std::map buckets, its GPU path sorts). */
 int sq_set_group_strategy(int strategy);
 int sq_get_group_strategy(int* strategy);

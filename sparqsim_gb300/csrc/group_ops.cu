@@ -445,7 +445,7 @@ struct EmitArgs {
     unsigned long long* ticket;  // dynamic group order: next group, CTAs finished (zero between launches)
     unsigned* err;               // device error word
     unsigned* glist;             // groups left by a singleton fan-out, and their number (glist_n);
-    unsigned* glist_n;           // emit_hadamard_kernel then runs over these groups only
+    unsigned* glist_n;           // emit_tile_kernel or emit_hadamard_kernel then runs over these groups only
 };
 
 // Dynamic group order for the persistent emit kernels. A grid of two CTAs
@@ -862,7 +862,7 @@ __global__ void __launch_bounds__(256) emit_fanout_kernel(const __grid_constant_
             }
         }
         // a group of several members (a few collisions among mostly singleton
-        // groups) is listed for emit_hadamard_kernel; without a list it only
+        // groups) is listed for the kernel launched after it; without a list it only
         // arises in a graph replayed on other data: nothing is written for it
         // and the replay is reported
         const bool one = valid && m == 1u;
@@ -1971,9 +1971,9 @@ __global__ void __launch_bounds__(512, 2) emit_h4096x_kernel(const __grid_consta
 // The warp-per-group kernel (emit_hadamard_kernel) keeps the slots in shared
 // memory: two reads and two writes per butterfly, half of the lanes idle on 16
 // members. The merges of 4096 batched instances of 4 to 8 bits (71 M entries
-// each): 733 us there, 496 here, now bound by integer issue (the ALU pipe 64 %
-// busy; about 2000 instructions per tile, of which 340 convert to the grid and
-// 256 are the butterflies). Also measured: rows unrolled (instruction cache
+// each): 733 us there, 496 here, now bound by integer issue (1024 instances: 58 %
+// issue, the ALU pipe 57 % busy, DRAM 20 %; about 2000 instructions per tile, of
+// which 340 convert to the grid and 256 are the butterflies). Also measured: rows unrolled (instruction cache
 // misses, 970 us), 3 CTAs of 8 warps at 80 registers (530 us), a copy for 8-bit
 // tiles with the width known to the compiler (508 us).
 constexpr unsigned kTileWarps = 4;    // per CTA
@@ -2841,7 +2841,7 @@ __global__ void __launch_bounds__(256) bucket_kernel(HashWs h, const uint64_t* _
 }  // namespace
 
 #ifndef SQ_GROUP_K
-static int g_strategy = 3;  // 0 heuristic (hash from 4096 entries), 1 sort, 2 hash, 3 autotuned
+static int g_strategy = 3;  // 0 automatic (hash), 1 sort, 2 hash, 3 autotuned
 static int g_sizing = 0;    // 0 auto (single pass when the output bound fits), 1 exact count-then-scan
 void set_output_sizing(int m) {
     if (m < 0 || m > 1) fail(SQ_ERR_INVALID, "output sizing must be 0 (auto) or 1 (count then scan)");
@@ -3557,7 +3557,7 @@ __global__ void __launch_bounds__(256) pair_scatter_kernel(ConstKeyPtrs keys, ui
 // and its threads take the list's items, so that no FP64 lane idles for an
 // entry whose partner does the work. ITEMS entries per thread keep their
 // lookups in flight together. Bound by the chain key, slot, partner's key,
-// amplitudes (36 % issue, FP64 pipe 23 %), so CTAs in flight count: four
+// amplitudes (36 % issue, FP64 pipe 41 %), so CTAs in flight count: four
 // entries per thread at 64 registers 56 us, two at 40 registers 49 (2^21
 // entries); writing each target value's outputs as a run of its own: 56.
 template <int K, int ITEMS>

@@ -1,6 +1,6 @@
-"""Entries read on another stream right after an operator has returned: entry
-points that return sizes have written their outputs by then. Elementwise
-operators, which return none, are not waited for."""
+"""Entries read on another stream right after a call has returned: ClearZero,
+1-bit splits, new and reset states have stored theirs by then. Elementwise
+operators, which return no size, are not waited for."""
 from __future__ import annotations
 
 import ctypes
