@@ -80,7 +80,9 @@ constexpr unsigned long long kCzUnchanged = 1ull << 63;
 // key selection accepts. Same single pass either way. any: prune_any's word
 // (null: compact whatever it would say); the number of survivors, or n |
 // kCzUnchanged when nothing was written, is posted to the host, by the CTA that
-// finishes last: the host returns to a caller who may read the entries.
+// finishes last: the host returns to a caller who may read the entries (3 us
+// more per call on 2^20 entries of two words than posting with the count, 44
+// against 47).
 template <int K, bool SEL>
 __global__ void __launch_bounds__(kCzBlock) clearzero_kernel(ConstKeyPtrs ik, const double2* __restrict__ ia,
                                                              KeyPtrs ok, double2* __restrict__ oa, uint64_t n,
